@@ -1107,15 +1107,17 @@ int cta_batch_solve(std::vector<Handle*>& hs, const gg_uzawa_params& prm, double
     for (int i = 0; i < n; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return hs[a]->nel > hs[b]->nel; });
     GG_CUDA(cudaDeviceSynchronize());  // every handle's build (own streams) is complete
-    // one device block for the descriptors, the order, the queue head and the outputs
+    // one device block for the descriptors, the outputs, the order and the queue head; the
+    // parts that hold 8-byte words come first, so an odd problem count misaligns none of them
     const size_t bp = sizeof(CtaProblem) * n, bo = sizeof(int32_t) * n, bs = sizeof(gg_uzawa_stats) * n;
     char* dev = nullptr;
     GG_CUDA(cudaMalloc(&dev, bp + bo + bs + sizeof(int32_t) * n + 256));
     CtaProblem* d_probs = reinterpret_cast<CtaProblem*>(dev);
-    int32_t* d_order = reinterpret_cast<int32_t*>(dev + bp);
-    gg_uzawa_stats* d_stats = reinterpret_cast<gg_uzawa_stats*>(dev + bp + bo);
-    int32_t* d_status = reinterpret_cast<int32_t*>(dev + bp + bo + bs);
-    int* d_next = reinterpret_cast<int*>(dev + bp + bo + bs + sizeof(int32_t) * n);
+    static_assert(sizeof(CtaProblem) % 8 == 0 && sizeof(gg_uzawa_stats) % 8 == 0, "batch block layout");
+    gg_uzawa_stats* d_stats = reinterpret_cast<gg_uzawa_stats*>(dev + bp);
+    int32_t* d_order = reinterpret_cast<int32_t*>(dev + bp + bs);
+    int32_t* d_status = reinterpret_cast<int32_t*>(dev + bp + bs + bo);
+    int* d_next = reinterpret_cast<int*>(dev + bp + bs + bo + sizeof(int32_t) * n);
     for (int i = 0; i < n; i++) {
         probs[i].stats = d_stats + i;
         probs[i].status = d_status + i;
