@@ -10,13 +10,16 @@
 //     rebuilds its boundary list from the neighbours (S, N, E, W, U, D) of the cells it
 //     just took that it does not own; passes repeat until one claims nothing;
 //   * centroid of i = mean centre of its cells, weight = cells × cell volume.
-// B200 mapping: one warp per element, the grid and the boundary lists in shared memory.
-// The points stay sequential, as in the reference, but within one point's turn the
-// claims and the boundary are sets: a cell's claim depends only on its current owner, and
-// the boundary is the set of neighbours of the new claims not owned by the point.  So a
-// point's turn runs across the 32 lanes (ballot compaction, a per-turn stamp
-// deduplicates the boundary) and gives the reference's ownership exactly.  Centroids are
-// summed per point in grid-cell order (one lane per point), the reference's order.
+// B200 mapping: the points of an element stay sequential, as in the reference, but within
+// one point's turn the claims and the boundary are sets: a cell's claim depends only on its
+// current owner, and the boundary is the set of neighbours of the new claims not owned by
+// the point.  So a point's turn runs across lanes (ballot compaction) and gives the
+// reference's ownership exactly.  Centroids are summed per point in grid-cell order, the
+// reference's order.
+// Two kernels share the work.  k_dvc_group takes the elements of up to 64 points whose
+// boundary lists stay within its ring, which is nearly every element of a run; the few it
+// cannot hold go to a list that k_dvc (one warp per element, room for 254 points and the
+// longest lists) finishes, errors included.
 //
 // Population control (lane 0, a few dozen items per element): the split list in list
 // order; the delete list sorted by decreasing point index; the limits and the interface
@@ -281,12 +284,8 @@ __device__ bool dvc_warp(const DvcArgs& a, DvcSmem& S, int n, int64_t e) {
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(32 * kWarps) k_dvc(DvcArgs a) {
-    extern __shared__ unsigned char smem_raw[];
-    DvcSmem& S = reinterpret_cast<DvcSmem*>(smem_raw)[threadIdx.x >> 5];
+__device__ void dvc_element(const DvcArgs& a, DvcSmem& S, int64_t e) {
     const int lane = threadIdx.x & 31;
-    const int64_t e = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
-    if (e >= a.nel) return;
     const int32_t off = a.offsets[e];
     const int n = a.offsets[e + 1] - off;
     if (a.pc && lane == 0) {
@@ -394,6 +393,494 @@ __global__ void __launch_bounds__(32 * kWarps) k_dvc(DvcArgs a) {
             a.new_w[q] = w;
         }
     }
+}
+
+// the elements k_dvc_group deferred: defer[0] of them, from defer[1]
+template <int DIM>
+__global__ void __launch_bounds__(32 * kWarps) k_dvc(DvcArgs a, const int32_t* __restrict__ defer) {
+    extern __shared__ unsigned char smem_raw[];
+    DvcSmem& S = reinterpret_cast<DvcSmem*>(smem_raw)[threadIdx.x >> 5];
+    const int32_t count = defer[0];
+    for (int32_t q = (int32_t)blockIdx.x * kWarps + (threadIdx.x >> 5); q < count; q += (int32_t)gridDim.x * kWarps) {
+        dvc_element<DIM>(a, S, defer[1 + q]);
+        __syncwarp();
+    }
+}
+
+// ---- small elements: G lanes per element ---------------------------------------------
+// What bounds the diagrams is the latency of one point's turn (a few dependent
+// shared-memory reads and ballots) times some 200 turns per element, so the time is set by
+// how many elements an SM has in flight.  Here an element takes 2 KB (2D) to 5 KB (3D) of
+// shared memory instead of 36 KB: the boundary lists of successive turns are one ring (a
+// turn's list is consumed before its successor is appended), its claimed cells overwrite
+// the consumed entries, the deduplication is a bitmap cleared after the turn, the points
+// with a list to contest are one 64-bit mask, and a counting sort of the cells by owner
+// (in the ring's memory) replaces a scan of all cells per centroid.  One warp per element
+// with 36 KB each kept 6 elements per SM: 22.4 ms for 32³ elements of 27 points on 10³
+// cells and 4.81 ms for 256×64 of 40 points on 10².  Now 2.34 ms (36 warps per SM, 84 % of
+// the issue slots used: bound by instruction issue) and 0.363 ms.
+// A warp holds 32/G elements that take their turns in lockstep.  A 2D list is a few cells
+// long and a 3D one a few tens, which is where the lanes per element come from: G = 8 / 16 /
+// 32 took 4.37 / 2.51 / 2.34 ms in 3D and 0.338 / 0.363 / 0.583 ms in 2D at 10² cells (16
+// is kept there for finer grids, whose lists are longer).
+struct DvcGroup {
+    int cap;           // points an element may hold
+    int ring;          // ring entries, a power of two ≥ the grid cells
+    int xi_at, owner_at, mark_at, ring_at, len_at, list_at, stride;  // byte layout of an element
+    uint32_t mnx, mny; // ⌈65536/nx⌉, ⌈65536/ny⌉: c/nx = c·mnx >> 16 exactly for c < 1024, nx ≤ 64
+    int32_t* defer;    // [0] count, then the elements left to k_dvc
+};
+constexpr int kGroupPts = 64;       // points per element: one 64-bit mask
+constexpr int kGroupThreads = 128;
+constexpr int kGroupPasses = 1024;
+
+template <int DIM>
+__device__ __forceinline__ void cell_ijk(const DvcArgs& a, const DvcGroup& f, int c, int& i, int& j, int& k) {
+    const int t = (int)(((uint32_t)c * f.mnx) >> 16);
+    i = c - t * a.nx;
+    k = DIM == 3 ? (int)(((uint32_t)t * f.mny) >> 16) : 0;
+    j = DIM == 3 ? t - k * a.ny : t;
+}
+
+template <int DIM>
+__device__ __forceinline__ int cell_neighbour(const DvcArgs& a, const DvcGroup& f, int c, int q) {
+    int i, j, k;
+    cell_ijk<DIM>(a, f, c, i, j, k);
+    const int ax = q >> 1, step = (q & 1) ? 1 : -1;
+    const int at = ax == 0 ? i : ax == 1 ? j : k, end = ax == 0 ? a.nx : ax == 1 ? a.ny : a.nz;
+    if ((unsigned)(at + step) >= (unsigned)end) return -1;
+    return c + step * (ax == 0 ? 1 : ax == 1 ? a.nx : a.nx * a.ny);
+}
+
+// One element's working set in shared memory.
+struct GroupMem {
+    double* xi;        // [DIM][cap]
+    uint8_t* owner;    // [ncell]
+    uint32_t* mark;    // [ncell/32] bitmap
+    uint16_t* ring;    // boundary lists; afterwards the cells sorted by owner
+    uint16_t* len;     // [cap] list lengths; afterwards the cells' first position per point
+    uint16_t* cnt;     // [cap] cells per point
+};
+
+// Diagram of the n points of every group of the warp (n = 0: the group idles).  False when
+// the element has to go to k_dvc.  On success M.cnt, M.len (first position) and M.ring (the
+// cells in order, grouped by owner) describe it.  All 32 lanes call it.
+template <int DIM, int G>
+__device__ __forceinline__ bool dvc_grow(const DvcArgs& a, const DvcGroup& f, const GroupMem& M, const double* cx,
+                                         const double* cy, const double* cz, int n) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr unsigned kGroupMask = G == 32 ? kFull : (1u << (G & 31)) - 1u;
+    constexpr int NQ = 2 * DIM;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), gsh = lane & ~(G - 1);
+    const unsigned below = (1u << gl) - 1u;
+    const uint32_t rmask = (uint32_t)f.ring - 1u;
+    const int words = (a.ncell + 3) >> 2, mwords = (a.ncell + 31) >> 5;
+    for (int w = gl; w < words; w += G) reinterpret_cast<uint32_t*>(M.owner)[w] = 0xffffffffu;
+    for (int w = gl; w < mwords; w += G) M.mark[w] = 0u;
+    __syncwarp();
+    // seeds: every point its cell, the later point where two share one; its first list is
+    // every neighbour of that cell (DVCWeights.cxx:693-725)
+    uint32_t head = 0, tail = 0;
+    uint64_t live = 0;
+    for (int base = 0; __any_sync(kFull, base < n); base += G) {
+        const int i = base + gl;
+        int c = 0, ci = 0, cj = 0, ck = 0, m = 0;
+        const bool have = i < n;
+        if (have) {
+            ci = __double2int_rz(__ddiv_rn(__dsub_rn(M.xi[i], -1.0), a.dx));
+            cj = __double2int_rz(__ddiv_rn(__dsub_rn(M.xi[f.cap + i], -1.0), a.dy));
+            ck = DIM == 3 ? __double2int_rz(__ddiv_rn(__dsub_rn(M.xi[2 * f.cap + i], -1.0), a.dz)) : 0;
+            ci = min(max(ci, 0), a.nx - 1);
+            cj = min(max(cj, 0), a.ny - 1);
+            ck = min(max(ck, 0), a.nz - 1);
+            c = ci + a.nx * (cj + a.ny * ck);
+            m = (cj > 0) + (cj < a.ny - 1) + (ci < a.nx - 1) + (ci > 0);
+            if (DIM == 3) m += (ck > 0) + (ck < a.nz - 1);
+        }
+        int incl = m;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, incl, o, G);
+            if (gl >= o) incl += t;
+        }
+        if (have) {
+            uint32_t pos = tail + incl - m;
+#pragma unroll
+            for (int q = 0; q < NQ; q++) {
+                const int nb = cell_neighbour<DIM>(a, f, c, q);
+                if (nb >= 0) M.ring[pos++ & rmask] = (uint16_t)nb;
+            }
+            M.len[i] = (uint16_t)m;
+        }
+        const unsigned b = (__ballot_sync(kFull, have && m > 0) >> gsh) & kGroupMask;
+        live |= (uint64_t)b << base;
+        tail += __shfl_sync(kFull, incl, G - 1, G);
+        // batches ascend, so only lanes of this batch compete: the highest index stays
+        if (have) M.owner[c] = (uint8_t)i;
+        __syncwarp();
+        while (__any_sync(kFull, have && M.owner[c] < i)) {
+            if (have && M.owner[c] < i) M.owner[c] = (uint8_t)i;
+            __syncwarp();
+        }
+    }
+    bool done = n == 0, ok = true;
+    uint64_t next = 0;
+    int claimed_pass = 0, pass = 0;
+    for (;;) {
+        if (!done && live == 0) {  // the pass is over: another one if it claimed anything
+            if (claimed_pass == 0 || next == 0) {
+                done = true;
+            } else if (++pass >= kGroupPasses) {
+                done = true;
+                ok = false;
+            } else {
+                live = next;
+                next = 0;
+                claimed_pass = 0;
+            }
+        }
+        if (__all_sync(kFull, done)) break;
+        const int i = done ? -1 : __ffsll((long long)live) - 1;
+        const int len = done ? 0 : M.len[i];
+        if (!done) live &= live - 1;
+        // contest the list (ClaimCells, DVCWeights.cxx:260-330)
+        int nclaim = 0;
+        for (int base = 0; __any_sync(kFull, base < len); base += G) {
+            const int k = base + gl;
+            bool take = false;
+            int c = 0;
+            if (k < len) {
+                c = M.ring[(head + k) & rmask];
+                const int o = M.owner[c];
+                if (o == kNone) {
+                    take = true;
+                } else if (o != i) {
+                    int ii, jj, kk;
+                    cell_ijk<DIM>(a, f, c, ii, jj, kk);
+                    const double c0[3] = {cx[ii], cy[jj], DIM == 3 ? cz[kk] : 0.0};
+                    double p1[3], p2[3];
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) {
+                        p1[d] = M.xi[d * f.cap + o];
+                        p2[d] = M.xi[d * f.cap + i];
+                    }
+                    take = dist_test<DIM>(c0, p1, p2) > 0.0;
+                }
+            }
+            const unsigned b = (__ballot_sync(kFull, take) >> gsh) & kGroupMask;
+            if (take) {
+                M.owner[c] = (uint8_t)i;
+                M.ring[(head + nclaim + __popc(b & below)) & rmask] = (uint16_t)c;
+            }
+            nclaim += __popc(b);
+        }
+        __syncwarp();
+        // the new list (UpdateBchain, DVCWeights.cxx:420-470): one lane per (claim, side)
+        int m = 0;
+        const int items = nclaim * NQ;
+        for (int base = 0; __any_sync(kFull, base < items); base += G) {
+            const int it = base + gl;
+            bool add = false;
+            int nb = -1;
+            if (it < items) {
+                nb = cell_neighbour<DIM>(a, f, M.ring[(head + it / NQ) & rmask], it % NQ);
+                if (nb >= 0 && M.owner[nb] != i) {
+                    const uint32_t bit = 1u << (nb & 31);
+                    add = !(atomicOr(&M.mark[nb >> 5], bit) & bit);
+                }
+            }
+            const unsigned b = (__ballot_sync(kFull, add) >> gsh) & kGroupMask;
+            if (add) {
+                const uint32_t pos = tail + m + __popc(b & below);
+                if (pos - head < (uint32_t)f.ring) M.ring[pos & rmask] = (uint16_t)nb;
+            }
+            m += __popc(b);
+        }
+        if (tail + m - head > (uint32_t)f.ring) {  // k_dvc has the room
+            done = true;
+            ok = false;
+            m = 0;
+        }
+        __syncwarp();
+        for (int k = gl; k < m; k += G) M.mark[M.ring[(tail + k) & rmask] >> 5] = 0u;
+        if (i >= 0) {
+            if (gl == 0) M.len[i] = (uint16_t)m;
+            head += len;
+            tail += m;
+            claimed_pass += nclaim;
+            if (m) next |= 1ull << i;
+        }
+        __syncwarp();
+    }
+    // cells per point, then the cells in order grouped by point
+    if (!ok) n = 0;
+    for (int i = gl; i < n; i += G) M.cnt[i] = 0;
+    __syncwarp();
+    bool unowned = false;
+    for (int base = 0; base < a.ncell; base += G) {
+        const int c = base + gl;
+        int o = kNone;
+        if (n && c < a.ncell) {
+            o = M.owner[c];
+            unowned |= o == kNone;
+        }
+        const unsigned peers = __match_any_sync(kFull, o | (gsh << 8));
+        if (o != kNone && (peers & ((1u << lane) - 1u)) == 0u) M.cnt[o] += (uint16_t)__popc(peers);
+        __syncwarp();
+    }
+    if ((__ballot_sync(kFull, unowned) >> gsh) & kGroupMask) {  // k_dvc reports it
+        ok = false;
+        n = 0;
+    }
+    int first = 0;
+    for (int base = 0; __any_sync(kFull, base < n); base += G) {
+        const int i = base + gl;
+        const int v = i < n ? M.cnt[i] : 0;
+        int incl = v;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, incl, o, G);
+            if (gl >= o) incl += t;
+        }
+        if (i < n) M.len[i] = (uint16_t)(first + incl - v);
+        first += __shfl_sync(kFull, incl, G - 1, G);
+    }
+    __syncwarp();
+    for (int base = 0; base < a.ncell; base += G) {
+        const int c = base + gl;
+        const int o = n && c < a.ncell ? M.owner[c] : kNone;
+        const unsigned peers = __match_any_sync(kFull, o | (gsh << 8));
+        const int at = o != kNone ? M.len[o] : 0;
+        __syncwarp();
+        if (o != kNone) {
+            const unsigned before = peers & ((1u << lane) - 1u);
+            M.ring[at + __popc(before)] = (uint16_t)c;
+            if (before == 0u) M.len[o] = (uint16_t)(at + __popc(peers));
+        }
+        __syncwarp();
+    }
+    return ok;
+}
+
+// centroid of point p (GetCentroids, DVCWeights.cxx:202-230): its cells in grid order;
+// M.len[p] is one past its last cell
+template <int DIM>
+__device__ __forceinline__ void dvc_centroid(const DvcArgs& a, const DvcGroup& f, const GroupMem& M, const double* cx,
+                                             const double* cy, const double* cz, int p, double* s) {
+    s[0] = s[1] = s[2] = 0.0;
+    const int cnt = M.cnt[p], b = M.len[p] - cnt;
+    for (int k = 0; k < cnt; k++) {
+        int i, j, l;
+        cell_ijk<DIM>(a, f, M.ring[b + k], i, j, l);
+        s[0] = __dadd_rn(s[0], cx[i]);
+        s[1] = __dadd_rn(s[1], cy[j]);
+        if (DIM == 3) s[2] = __dadd_rn(s[2], cz[l]);
+    }
+    if (cnt) {
+#pragma unroll
+        for (int d = 0; d < DIM; d++) s[d] = __ddiv_rn(s[d], (double)cnt);
+    }
+}
+
+template <int DIM, int G>
+__global__ void __launch_bounds__(kGroupThreads) k_dvc_group(DvcArgs a, DvcGroup f) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double cx[kAxis], cy[kAxis], cz[kAxis];
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    // cell centres by the grid constructor's repeated additions (DVCWeights.cxx:557-575)
+    if (threadIdx.x < 3) {
+        double* out = threadIdx.x == 0 ? cx : threadIdx.x == 1 ? cy : cz;
+        const double dd = threadIdx.x == 0 ? a.dx : threadIdx.x == 1 ? a.dy : a.dz;
+        const int m = threadIdx.x == 0 ? a.nx : threadIdx.x == 1 ? a.ny : a.nz;
+        double X = __dsub_rn(-1.0, __ddiv_rn(dd, 2.0));
+        for (int i = 0; i < m; i++) out[i] = X = __dadd_rn(X, dd);
+    }
+    __syncthreads();
+    unsigned char* base = smem_raw + (size_t)(threadIdx.x / G) * f.stride;
+    GroupMem M;
+    M.xi = reinterpret_cast<double*>(base + f.xi_at);
+    M.owner = base + f.owner_at;
+    M.mark = reinterpret_cast<uint32_t*>(base + f.mark_at);
+    M.ring = reinterpret_cast<uint16_t*>(base + f.ring_at);
+    M.len = reinterpret_cast<uint16_t*>(base + f.len_at);
+    M.cnt = M.len + f.cap;
+    int8_t* list = reinterpret_cast<int8_t*>(base + f.list_at);  // point, or −1 − s for split s
+    uint8_t* split = reinterpret_cast<uint8_t*>(list) + f.cap;
+    uint8_t* del = split + f.cap;
+    const int64_t e = (int64_t)blockIdx.x * (kGroupThreads / G) + threadIdx.x / G;
+    const bool own = e < a.nel;
+    const int32_t off = own ? a.offsets[e] : 0;
+    int n = own ? a.offsets[e + 1] - off : 0;
+    if (own && a.pc && gl == 0) {
+        a.nsplit[e] = 0;
+        a.ndel[e] = 0;
+    }
+    bool defer = n + (a.pc ? a.max_splits : 0) > f.cap;
+    if (defer) n = 0;
+    for (int i = gl; i < n; i += G) {
+#pragma unroll
+        for (int d = 0; d < DIM; d++) M.xi[d * f.cap + i] = a.xi_s[(int64_t)d * a.np + off + i];
+        if (a.pc) list[i] = (int8_t)i;
+    }
+    __syncwarp();
+    if (!dvc_grow<DIM, G>(a, f, M, cx, cy, cz, n)) {
+        defer = true;
+        n = 0;
+    }
+    int m = n, nsplit = 0;
+    if (a.pc) {
+        // decisions (PCDVC.cxx:940-1013): the group's first lane
+        bool mixed = false;
+        const int m0 = n ? a.mat_s[off] : 0;
+        for (int i = gl; i < n; i += G) mixed |= a.mat_s[off + i] != m0;
+        const unsigned mb = __ballot_sync(kFull, mixed) >> (lane & ~(G - 1));
+        mixed = (mb & (G == 32 ? kFull : (1u << (G & 31)) - 1u)) != 0u;
+        int ndel = 0;
+        if (gl == 0 && n) {
+            const int maxS = mixed && !a.split_if ? 0 : a.max_splits;
+            int maxD = mixed && !a.delete_if ? 0 : a.max_deletions;
+            int ns = 0, nd = 0;
+            for (int i = 0; i < n; i++) {
+                const double w = __dmul_rn((double)M.cnt[i], a.da);
+                if (w > a.maxW && ns < maxS) split[ns++] = (uint8_t)i;
+                if (w < a.minW) del[nd++] = (uint8_t)i;
+            }
+            if (maxD > n - 4) maxD = n / 2;
+            nsplit = ns;
+            ndel = maxD > nd ? nd : maxD;
+            if (ndel > 0)
+                for (int x = 1; x < nd; x++)  // decreasing point index
+                    for (int y = x; y > 0 && a.perm[off + del[y - 1]] < a.perm[off + del[y]]; y--) {
+                        const uint8_t tmp = del[y];
+                        del[y] = del[y - 1];
+                        del[y - 1] = tmp;
+                    }
+            // new points: appended, at their parent's centroid
+            for (int s = 0; s < nsplit; s++) {
+                double cc[3];
+                dvc_centroid<DIM>(a, f, M, cx, cy, cz, split[s], cc);
+                list[m] = (int8_t)(-1 - s);
+#pragma unroll
+                for (int d = 0; d < DIM; d++) M.xi[d * f.cap + m] = cc[d];
+                m++;
+            }
+            // deletions: the list's last entry takes the deleted entry's place
+            for (int q = 0; q < ndel; q++) {
+                int pos = 0;
+                for (int k = 0; k < m; k++)
+                    if (list[k] == (int8_t)del[q]) pos = k;
+                list[pos] = list[m - 1];
+#pragma unroll
+                for (int d = 0; d < DIM; d++) M.xi[d * f.cap + pos] = M.xi[d * f.cap + m - 1];
+                m--;
+            }
+            if ((m != n || nsplit) && m < 3) defer = true;  // k_dvc reports it
+        }
+        __syncwarp();
+        m = __shfl_sync(kFull, m, 0, G);
+        nsplit = __shfl_sync(kFull, nsplit, 0, G);
+        ndel = __shfl_sync(kFull, ndel, 0, G);
+        defer = __shfl_sync(kFull, (int)defer, 0, G);
+        const bool again = !defer && (nsplit || ndel);
+        if (__any_sync(kFull, again)) {
+            // groups without a change keep their diagram: they sit the second growth out
+            // with a copy of nothing, so their results are written first
+            if (!again && !defer) {
+                for (int k = gl; k < m; k += G) {
+                    double cc[3];
+                    dvc_centroid<DIM>(a, f, M, cx, cy, cz, k, cc);
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) a.cent_out[(int64_t)d * a.np + off + k] = cc[d];
+                    a.w_out[off + k] = __dmul_rn((double)M.cnt[k], a.da);
+                }
+                m = 0;
+            }
+            __syncwarp();
+            if (!dvc_grow<DIM, G>(a, f, M, cx, cy, cz, again ? m : 0)) defer = true;
+        }
+        if (!defer && ndel)
+            for (int q = gl; q < ndel; q += G) a.keep[off + del[q]] = 0;
+        if (!defer && own && gl == 0) {
+            a.nsplit[e] = nsplit;
+            a.ndel[e] = ndel;
+        }
+    }
+    if (defer) {
+        if (own && gl == 0) f.defer[1 + atomicAdd(&f.defer[0], 1)] = (int32_t)e;
+        return;
+    }
+    for (int k = gl; k < m; k += G) {
+        const int src = a.pc ? list[k] : k;
+        const double w = __dmul_rn((double)M.cnt[k], a.da);
+        double cc[3];
+        dvc_centroid<DIM>(a, f, M, cx, cy, cz, k, cc);
+        if (src >= 0) {
+            const int64_t i = off + src;
+#pragma unroll
+            for (int d = 0; d < DIM; d++) a.cent_out[(int64_t)d * a.np + i] = cc[d];
+            a.w_out[i] = w;
+        } else {
+            const int s = -1 - src;
+            const int64_t q = e * a.stride + s;
+            a.new_parent[q] = off + split[s];
+#pragma unroll
+            for (int d = 0; d < DIM; d++) {
+                a.new_xi[q * DIM + d] = M.xi[d * f.cap + k];
+                a.new_cent[q * DIM + d] = cc[d];
+            }
+            a.new_w[q] = w;
+        }
+    }
+}
+
+template <int DIM, int G>
+void launch_group(const DvcArgs& a, DvcGroup f, int cap, cudaStream_t st) {
+    int at = 0;
+    auto take = [&](int bytes, int align) {
+        at = (at + align - 1) / align * align;
+        const int r = at;
+        at += bytes;
+        return r;
+    };
+    f.cap = cap;
+    int r = 32;
+    while (r < a.ncell || r < 2 * DIM * cap || (r < 2 * a.ncell && r < 512)) r *= 2;
+    f.ring = r;
+    f.xi_at = take((int)sizeof(double) * DIM * cap, 16);
+    f.mark_at = take((a.ncell + 31) / 32 * 4, 4);
+    f.owner_at = take((a.ncell + 3) / 4 * 4, 4);
+    f.ring_at = take(2 * r, 2);
+    f.len_at = take(4 * cap, 2);
+    f.list_at = take(a.pc ? 3 * cap : 0, 1);
+    f.stride = (at + 15) / 16 * 16 + 16;  // the odd 16 bytes spread the groups over the banks
+    f.mnx = (65536u + a.nx - 1) / a.nx;
+    f.mny = (65536u + a.ny - 1) / a.ny;
+    constexpr int per = kGroupThreads / G;
+    const size_t smem = (size_t)f.stride * per;
+    GG_CUDA(cudaFuncSetAttribute(k_dvc_group<DIM, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_dvc_group<DIM, G><<<(unsigned)((a.nel + per - 1) / per), kGroupThreads, smem, st>>>(a, f);
+    GG_CUDA(cudaGetLastError());
+}
+
+// Every element through k_dvc_group, the deferred ones through k_dvc.
+template <int DIM>
+void launch_dvc(const DvcArgs& a, int32_t* defer, cudaStream_t st) {
+    GG_CUDA(cudaMemsetAsync(defer, 0, sizeof(int32_t), st));
+    // room for half again the mean point count: uniform swarms and those PCDVC keeps within
+    // its bounds stay below it, and smaller elements leave room for more of them per SM
+    const double mean = (double)a.np / (double)a.nel;
+    int cap = ((int)(1.5 * mean) + 8 + 7) / 8 * 8;
+    cap = cap > kGroupPts ? kGroupPts : cap;
+    DvcGroup f{};
+    f.defer = defer;
+    launch_group<DIM, DIM == 3 ? 32 : 16>(a, f, cap, st);
+    const size_t smem = sizeof(DvcSmem) * kWarps;
+    GG_CUDA(cudaFuncSetAttribute(k_dvc<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int64_t want = (a.nel + kWarps - 1) / kWarps;
+    const int blocks = (int)std::min<int64_t>(want, 2 * num_sms());
+    k_dvc<DIM><<<blocks, 32 * kWarps, smem, st>>>(a, defer);
+    GG_CUDA(cudaGetLastError());
 }
 
 // ---- rebuilding the point set after population control ------------------------------
@@ -580,16 +1067,11 @@ int dvc_update(Handle& H, const gg_pcdvc_params* prm, gg_pcdvc_stats* stats) {
         a.nsplit = H.dvc_nsplit.as<int32_t>();
         a.ndel = H.dvc_ndel.as<int32_t>();
     }
-    const size_t smem = sizeof(DvcSmem) * kWarps;
-    const int blocks = (int)((nel + kWarps - 1) / kWarps);
-    if (dim == 2) {
-        GG_CUDA(cudaFuncSetAttribute(k_dvc<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_dvc<2><<<blocks, 32 * kWarps, smem, st>>>(a);
-    } else {
-        GG_CUDA(cudaFuncSetAttribute(k_dvc<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_dvc<3><<<blocks, 32 * kWarps, smem, st>>>(a);
-    }
-    GG_CUDA(cudaGetLastError());
+    H.dvc_defer.ensure(sizeof(int32_t) * (nel + 1));
+    if (dim == 2)
+        launch_dvc<2>(a, H.dvc_defer.as<int32_t>(), st);
+    else
+        launch_dvc<3>(a, H.dvc_defer.as<int32_t>(), st);
     int32_t err[2] = {0, 0};
     GG_CUDA(cudaMemcpyAsync(err, H.dvc_err.p, sizeof err, cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));
@@ -624,7 +1106,7 @@ int dvc_update(Handle& H, const gg_pcdvc_params* prm, gg_pcdvc_stats* stats) {
         return GG_OK;
     }
     // point order: keep flags, integration points
-    DBuf keep_p, newidx, xi_p, w_p;
+    DBuf &keep_p = H.pc_keep, &newidx = H.pc_newidx, &xi_p = H.pc_xi_p, &w_p = H.pc_w_p;
     keep_p.ensure(sizeof(int32_t) * np);
     newidx.ensure(sizeof(int32_t) * (np + 1));
     xi_p.ensure(sizeof(double) * np * dim);
@@ -635,7 +1117,7 @@ int dvc_update(Handle& H, const gg_pcdvc_params* prm, gg_pcdvc_stats* stats) {
     int32_t nsurv = 0;
     exclusive_scan_i32(H, keep_p.as<int32_t>(), newidx.as<int32_t>(), np, H.scan_tmp, &nsurv);
     const int64_t np2 = (int64_t)nsurv + nsplit_tot;
-    DBuf coords2, mat2, ps2, xi2, w2;
+    DBuf &coords2 = H.pc_coords, &mat2 = H.pc_mat, &ps2 = H.pc_ps, &xi2 = H.pc_xi, &w2 = H.pc_w;
     coords2.ensure(sizeof(double) * np2 * dim);
     mat2.ensure(sizeof(int32_t) * np2);
     ps2.ensure(sizeof(double) * np2);

@@ -91,7 +91,10 @@ struct Handle {
     // the material points' own ξ, from which the diagrams grow
     gg_weights weights{GG_WEIGHTS_CONSTANT, {10, 10, 10}};
     bool dvc_valid = false;
-    DBuf w_s, xi_pts, dvc_cent, dvc_keep, dvc_err, dvc_nsplit, dvc_ndel, dvc_parent, dvc_new, dvc_scan, dvc_scan2;
+    DBuf w_s, xi_pts, dvc_defer, dvc_cent, dvc_keep, dvc_err, dvc_nsplit, dvc_ndel, dvc_parent, dvc_new, dvc_scan, dvc_scan2;
+    // population control's point-order scratch and the other half of the point set it swaps in
+    DBuf pc_keep, pc_newidx, pc_xi_p, pc_w_p, pc_coords, pc_mat, pc_ps, pc_xi, pc_w;
+    DBuf int_xi, int_w;  // integration points in point order (gg_get_integration_points)
 
     // operator
     DBuf mom64, mom32, kdiag64, kdiag32, sdiag, hvec, f;

@@ -97,3 +97,36 @@ def test_population_control_statuses():
     assert e.value.code == -1
     with pytest.raises(GaleError):
         G.set_weights("dvc", 40)  # 40 × 40 > 1024 cells
+
+
+@pytest.mark.parametrize("dim,res,most", [(2, [10, 10], 90), (2, [64, 16], 64), (2, [3, 2], 20), (2, [1, 1], 3),
+                                          (3, [10, 10, 10], 64), (3, [4, 4, 64], 40), (3, [7, 5, 3], 30)])
+def test_dvc_weights_uneven_elements(oracle_mod, dim, res, most):
+    """Elements of 1 to `most` points (both kernels where more than 64), several in one grid
+    cell, some coincident (ties) or on cell faces: the oracle's diagrams bit for bit, grown
+    from the same local coordinates (points 1e-9 apart tell the oracle's Newton iterate of ξ
+    from its closed form, which the whole-mesh oracle call would compare as well)."""
+    rng = np.random.default_rng(dim * 100 + most)
+    mesh = Mesh(dim, [5] * dim)
+    cells = np.stack(np.meshgrid(*[np.arange(5)] * dim, indexing="ij"), -1).reshape(-1, dim)
+    pts = []
+    for c in cells:
+        t = rng.uniform(0.01, 0.99, (rng.integers(1, most + 1), dim))
+        if len(t) > 3:
+            t[1] = t[0]                          # coincident points
+            t[2] = t[0] + 1e-9                   # the same grid cell
+            t[3] = np.round(t[3] * 8) / 8 * 0.9 + 0.05
+        pts.append((c + t) / 5)
+    x = rng.permutation(np.concatenate(pts))
+    G = StokesProblem(mesh)
+    G.set_points(x, np.zeros(len(x), dtype=np.int32))
+    cell = G.locate()
+    local, _ = G.integration_points()
+    G.set_weights("dvc", res)
+    G.locate()
+    xi, wt = G.integration_points()
+    for e in range(5 ** dim):
+        idx = np.flatnonzero(cell == e)
+        cent, w_ref = oracle_mod.dvc_cell(dim, res, local[idx])
+        assert np.array_equal(wt[idx], w_ref)
+        assert np.array_equal(xi[idx], cent)
