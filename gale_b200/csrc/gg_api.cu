@@ -197,6 +197,7 @@ int gg_create(const gg_mesh_desc* mesh, gg_handle** out) {
         delete h;
         return GG_ERR_CUDA;
     }
+    gg::copy_handle_created();
     *out = h;
     return GG_OK;
 }
@@ -213,6 +214,7 @@ int gg_destroy(gg_handle* h) {
     if (H.evf1) cudaEventDestroy(H.evf1);
     if (H.stream) cudaStreamDestroy(H.stream);
     delete h;
+    gg::copy_handle_destroyed();
     return GG_OK;
 }
 
@@ -240,8 +242,8 @@ int gg_set_velocity_bc(gg_handle* h, const gg_velocity_bc* bc) {
             for (int c = 0; c < dim; c++) nfixed += (mask[n] >> c) & 1;
         }
         H.nfree = H.ndof - nfixed;
-        GG_CUDA(cudaMemcpyAsync(H.bcmask.p, mask.data(), H.nnode, cudaMemcpyHostToDevice, H.stream));
-        GG_CUDA(cudaMemcpyAsync(H.bcval.p, val.data(), sizeof(double) * H.ndof, cudaMemcpyHostToDevice, H.stream));
+        gg::copy_to_device(H, H.bcmask.p, mask.data(), H.nnode);
+        gg::copy_to_device(H, H.bcval.p, val.data(), sizeof(double) * H.ndof);
         GG_CUDA(cudaStreamSynchronize(H.stream));
         H.has_bc = true;
         H.built = false;
@@ -267,8 +269,8 @@ int gg_set_velocity_bc_nodes(gg_handle* h, const uint8_t* fixed, const double* v
                 }
         }
         H.nfree = H.ndof - nfixed;
-        GG_CUDA(cudaMemcpyAsync(H.bcmask.p, mask.data(), H.nnode, cudaMemcpyHostToDevice, H.stream));
-        GG_CUDA(cudaMemcpyAsync(H.bcval.p, val.data(), sizeof(double) * H.ndof, cudaMemcpyHostToDevice, H.stream));
+        gg::copy_to_device(H, H.bcmask.p, mask.data(), H.nnode);
+        gg::copy_to_device(H, H.bcval.p, val.data(), sizeof(double) * H.ndof);
         GG_CUDA(cudaStreamSynchronize(H.stream));
         H.has_bc = true;
         H.built = false;
@@ -317,13 +319,13 @@ int gg_set_points(gg_handle* h, int64_t n, const double* coords, const int32_t* 
         for (gg::DBuf* b : {&H.ps_s, &H.eta_s, &H.incr_s}) b->ensure(sizeof(double) * n);
         H.xi_s.ensure(sizeof(double) * n * dim);
         H.yld_s.ensure(n);
-        GG_CUDA(cudaMemcpyAsync(H.coords.p, coords, sizeof(double) * n * dim, cudaMemcpyHostToDevice, H.stream));
+        gg::copy_to_device(H, H.coords.p, coords, sizeof(double) * n * dim);
         if (material)
-            GG_CUDA(cudaMemcpyAsync(H.mat_in.p, material, sizeof(int32_t) * n, cudaMemcpyHostToDevice, H.stream));
+            gg::copy_to_device(H, H.mat_in.p, material, sizeof(int32_t) * n);
         else
             GG_CUDA(cudaMemsetAsync(H.mat_in.p, 0, sizeof(int32_t) * n, H.stream));
         if (plastic_strain)
-            GG_CUDA(cudaMemcpyAsync(H.ps_in.p, plastic_strain, sizeof(double) * n, cudaMemcpyHostToDevice, H.stream));
+            gg::copy_to_device(H, H.ps_in.p, plastic_strain, sizeof(double) * n);
         else
             GG_CUDA(cudaMemsetAsync(H.ps_in.p, 0, sizeof(double) * n, H.stream));
         GG_CUDA(cudaStreamSynchronize(H.stream));
@@ -340,7 +342,7 @@ int gg_set_temperature(gg_handle* h, const double* T) {
     GG_TRY(h, {
         if (T) {
             H.T.ensure(sizeof(double) * H.nnode);
-            GG_CUDA(cudaMemcpyAsync(H.T.p, T, sizeof(double) * H.nnode, cudaMemcpyHostToDevice, H.stream));
+            gg::copy_to_device(H, H.T.p, T, sizeof(double) * H.nnode);
             GG_CUDA(cudaStreamSynchronize(H.stream));
             H.has_T = true;
         } else {
@@ -375,8 +377,7 @@ int gg_locate(gg_handle* h, uint32_t* owning_cell) {
         H.dvc_valid = false;
         if (!outside && H.weights.mode == GG_WEIGHTS_DVC) rc = gg::dvc_update(H, nullptr, nullptr);
         if (owning_cell) {
-            GG_CUDA(cudaMemcpyAsync(owning_cell, H.cell.p, sizeof(uint32_t) * H.np, cudaMemcpyDeviceToHost, H.stream));
-            GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, owning_cell, H.cell.p, sizeof(uint32_t) * H.np);
         }
     })
     H.located = outside == 0 && rc == GG_OK;
@@ -392,7 +393,7 @@ namespace gg {
 static void upload_nodal(Handle& H, const double* host, DBuf& dst, bool zero_bc) {
     H.ftmp.ensure(sizeof(double) * H.ndof);
     dst.ensure(sizeof(double) * H.ndof);
-    GG_CUDA(cudaMemcpyAsync(H.ftmp.p, host, sizeof(double) * H.ndof, cudaMemcpyHostToDevice, H.stream));
+    gg::copy_to_device(H, H.ftmp.p, host, sizeof(double) * H.ndof);
     k_nodal_to_soa<<<grid(H.ndof), 256, 0, H.stream>>>(H.nnode, H.dim, H.ftmp.as<double>(), H.bcmask.as<uint8_t>(),
                                                         zero_bc ? 1 : 0, dst.as<double>());
     GG_CUDA(cudaGetLastError());
@@ -401,15 +402,13 @@ static void download_nodal(Handle& H, const double* dsrc, const double* add, dou
     H.ftmp.ensure(sizeof(double) * H.ndof);
     k_soa_to_nodal<<<grid(H.ndof), 256, 0, H.stream>>>(H.nnode, H.dim, dsrc, add, H.ftmp.as<double>());
     GG_CUDA(cudaGetLastError());
-    GG_CUDA(cudaMemcpyAsync(host, H.ftmp.p, sizeof(double) * H.ndof, cudaMemcpyDeviceToHost, H.stream));
-    GG_CUDA(cudaStreamSynchronize(H.stream));
+    gg::copy_to_host(H, host, H.ftmp.p, sizeof(double) * H.ndof);
 }
 
 void download_solution(Handle& H, double* u, double* p) {
     store_solution(H);
     download_nodal(H, H.u.as<double>(), H.bcval.as<double>(), u);
-    GG_CUDA(cudaMemcpyAsync(p, H.q.p, sizeof(double) * H.nel, cudaMemcpyDeviceToHost, H.stream));
-    GG_CUDA(cudaStreamSynchronize(H.stream));
+    gg::copy_to_host(H, p, H.q.p, sizeof(double) * H.nel);
     H.have_solution = true;
 }
 
@@ -458,7 +457,7 @@ int gg_build_operator(gg_handle* h, int32_t precision, int32_t prev, const doubl
             du = H.prev_u.as<double>();
             if (p) {
                 H.prev_p.ensure(sizeof(double) * H.nel);
-                GG_CUDA(cudaMemcpyAsync(H.prev_p.p, p, sizeof(double) * H.nel, cudaMemcpyHostToDevice, H.stream));
+                gg::copy_to_device(H, H.prev_p.p, p, sizeof(double) * H.nel);
                 dp = H.prev_p.as<double>();
             }
         }
@@ -479,14 +478,13 @@ int gg_uzawa_solve(gg_handle* h, const gg_uzawa_params* prm, double* u, double* 
     gg_uzawa_stats S{};
     GG_TRY(h, {
         if (prm->reuse_pressure)
-            GG_CUDA(cudaMemcpyAsync(H.q.p, p, sizeof(double) * H.nel, cudaMemcpyHostToDevice, H.stream));
+            gg::copy_to_device(H, H.q.p, p, sizeof(double) * H.nel);
         else
             GG_CUDA(cudaMemsetAsync(H.q.p, 0, sizeof(double) * H.nel, H.stream));
         rc = gg::uzawa_solve(H, *prm, S);
         gg::store_solution(H);
         gg::download_nodal(H, H.u.as<double>(), H.bcval.as<double>(), u);
-        GG_CUDA(cudaMemcpyAsync(p, H.q.p, sizeof(double) * H.nel, cudaMemcpyDeviceToHost, H.stream));
-        GG_CUDA(cudaStreamSynchronize(H.stream));
+        gg::copy_to_host(H, p, H.q.p, sizeof(double) * H.nel);
         H.have_solution = true;
     })
     if (stats) *stats = S;

@@ -84,7 +84,7 @@ __global__ void k_diff_norms(int64_t n, const double* __restrict__ a, const doub
 
 void nodal_in(Handle& H, const double* host, double* dst, bool zero_bc) {
     H.ftmp.ensure(sizeof(double) * H.ndof);
-    GG_CUDA(cudaMemcpyAsync(H.ftmp.p, host, sizeof(double) * H.ndof, cudaMemcpyHostToDevice, H.stream));
+    gg::copy_to_device(H, H.ftmp.p, host, sizeof(double) * H.ndof);
     k_nodal_to_soa2<<<grid(H.ndof), 256, 0, H.stream>>>(H.nnode, H.dim, H.ftmp.as<double>(), H.bcmask.as<uint8_t>(),
                                                          zero_bc ? 1 : 0, dst);
     GG_CUDA(cudaGetLastError());
@@ -94,8 +94,7 @@ void nodal_out(Handle& H, const double* src, double* host) {
     H.ftmp.ensure(sizeof(double) * H.ndof);
     k_soa_to_nodal2<<<grid(H.ndof), 256, 0, H.stream>>>(H.nnode, H.dim, src, H.ftmp.as<double>());
     GG_CUDA(cudaGetLastError());
-    GG_CUDA(cudaMemcpyAsync(host, H.ftmp.p, sizeof(double) * H.ndof, cudaMemcpyDeviceToHost, H.stream));
-    GG_CUDA(cudaStreamSynchronize(H.stream));
+    gg::copy_to_host(H, host, H.ftmp.p, sizeof(double) * H.ndof);
 }
 
 int err(Handle& H, int code, const std::string& m) {
@@ -176,8 +175,7 @@ int gg_picard(gg_handle* h, const gg_picard_params* pic, const gg_uzawa_params* 
         }
         if (H.have_solution || rc == GG_OK) {
             gg::nodal_out(H, H.prev_u.as<double>(), u);
-            GG_CUDA(cudaMemcpyAsync(p, H.q.p, sizeof(double) * H.nel, cudaMemcpyDeviceToHost, H.stream));
-            GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, p, H.q.p, sizeof(double) * H.nel);
         }
         H.have_solution = rc == GG_OK;
     })
@@ -200,9 +198,7 @@ int gg_advect(gg_handle* h, double dt, int32_t order, const double* u, double* c
         }
         rc = gg::advect(H, dt, order, H.prev_u.as<double>(), nullptr);
         if (coords_out) {
-            GG_CUDA(cudaMemcpyAsync(coords_out, H.coords.p, sizeof(double) * H.np * H.dim, cudaMemcpyDeviceToHost,
-                                    H.stream));
-            GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, coords_out, H.coords.p, sizeof(double) * H.np * H.dim);
         }
     })
     if (rc != GG_OK) gg::err(H, rc, "a material point left the mesh in the predictor stage");
@@ -231,8 +227,7 @@ int gg_get_point_viscosity(gg_handle* h, double* eta) {
         H.ftmp.ensure(sizeof(double) * (H.np > H.ndof ? H.np : H.ndof));
         gg::k_unsort<double><<<grid(H.np_in), 256, 0, H.stream>>>(H.np_in, H.perm.as<int32_t>(), H.eta_s.as<double>(),
                                                                   H.ftmp.as<double>());
-        GG_CUDA(cudaMemcpyAsync(eta, H.ftmp.p, sizeof(double) * H.np, cudaMemcpyDeviceToHost, H.stream));
-        GG_CUDA(cudaStreamSynchronize(H.stream));
+        gg::copy_to_host(H, eta, H.ftmp.p, sizeof(double) * H.np);
     })
     return GG_OK;
 }
@@ -246,14 +241,12 @@ int gg_get_point_yield(gg_handle* h, double* increment, uint8_t* yielded) {
         if (increment) {
             gg::k_unsort<double><<<grid(H.np_in), 256, 0, H.stream>>>(H.np_in, H.perm.as<int32_t>(),
                                                                       H.incr_s.as<double>(), H.ftmp.as<double>());
-            GG_CUDA(cudaMemcpyAsync(increment, H.ftmp.p, sizeof(double) * H.np, cudaMemcpyDeviceToHost, H.stream));
-            GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, increment, H.ftmp.p, sizeof(double) * H.np);
         }
         if (yielded) {
             gg::k_unsort<uint8_t><<<grid(H.np_in), 256, 0, H.stream>>>(H.np_in, H.perm.as<int32_t>(),
                                                                        H.yld_s.as<uint8_t>(), H.ftmp.as<uint8_t>());
-            GG_CUDA(cudaMemcpyAsync(yielded, H.ftmp.p, H.np, cudaMemcpyDeviceToHost, H.stream));
-            GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, yielded, H.ftmp.p, H.np);
         }
     })
     return GG_OK;
@@ -266,8 +259,7 @@ int gg_get_moments(gg_handle* h, double* moments, int32_t* n_moments) {
     if (!moments) return GG_OK;
     if (!H.built) return gg::err(H, GG_ERR_STATE, "operator not built");
     GG_TRY2(h, {
-        GG_CUDA(cudaMemcpyAsync(moments, H.mom64.p, sizeof(double) * H.nm * H.nel, cudaMemcpyDeviceToHost, H.stream));
-        GG_CUDA(cudaStreamSynchronize(H.stream));
+        gg::copy_to_host(H, moments, H.mom64.p, sizeof(double) * H.nm * H.nel);
     })
     return GG_OK;
 }
@@ -421,12 +413,11 @@ int gg_get_points(gg_handle* h, double* coords, int32_t* material, double* plast
     if (H.np == 0) return gg::err(H, GG_ERR_STATE, "points not set");
     GG_TRY2(h, {
         if (coords)
-            GG_CUDA(cudaMemcpyAsync(coords, H.coords.p, sizeof(double) * H.np * H.dim, cudaMemcpyDeviceToHost, H.stream));
+            gg::copy_to_host(H, coords, H.coords.p, sizeof(double) * H.np * H.dim);
         if (material)
-            GG_CUDA(cudaMemcpyAsync(material, H.mat_in.p, sizeof(int32_t) * H.np, cudaMemcpyDeviceToHost, H.stream));
+            gg::copy_to_host(H, material, H.mat_in.p, sizeof(int32_t) * H.np);
         if (plastic_strain)
-            GG_CUDA(cudaMemcpyAsync(plastic_strain, H.ps_in.p, sizeof(double) * H.np, cudaMemcpyDeviceToHost, H.stream));
-        GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, plastic_strain, H.ps_in.p, sizeof(double) * H.np);
     })
     return GG_OK;
 }
@@ -465,9 +456,8 @@ int gg_get_integration_points(gg_handle* h, double* xi, double* weight) {
             H.weights.mode == GG_WEIGHTS_DVC && H.dvc_valid ? H.w_s.as<double>() : nullptr, dx.as<double>(),
             dw.as<double>());
         GG_CUDA(cudaGetLastError());
-        GG_CUDA(cudaMemcpyAsync(xi, dx.p, sizeof(double) * H.np * H.dim, cudaMemcpyDeviceToHost, H.stream));
-        GG_CUDA(cudaMemcpyAsync(weight, dw.p, sizeof(double) * H.np, cudaMemcpyDeviceToHost, H.stream));
-        GG_CUDA(cudaStreamSynchronize(H.stream));
+        gg::copy_to_host(H, xi, dx.p, sizeof(double) * H.np * H.dim);
+        gg::copy_to_host(H, weight, dw.p, sizeof(double) * H.np);
     })
     return GG_OK;
 }
@@ -550,7 +540,7 @@ int gg_apply_G(gg_handle* h, const double* p, double* y) {
     GG_TRY2(h, {
         H.qtmp.ensure(sizeof(double) * H.nel);
         H.ub.ensure(sizeof(double) * H.ndof);
-        GG_CUDA(cudaMemcpyAsync(H.qtmp.p, p, sizeof(double) * H.nel, cudaMemcpyHostToDevice, H.stream));
+        gg::copy_to_device(H, H.qtmp.p, p, sizeof(double) * H.nel);
         gg::apply_G(H, H.qtmp.as<double>(), H.ub.as<double>(), H.stream);
         gg::nodal_out(H, H.ub.as<double>(), y);
     })
@@ -565,8 +555,7 @@ int gg_apply_GT(gg_handle* h, const double* u, double* q) {
         H.vstar.ensure(sizeof(double) * H.ndof);
         gg::nodal_in(H, u, H.vstar.as<double>(), true);
         gg::apply_GT(H, H.vstar.as<double>(), H.qtmp.as<double>(), H.stream);
-        GG_CUDA(cudaMemcpyAsync(q, H.qtmp.p, sizeof(double) * H.nel, cudaMemcpyDeviceToHost, H.stream));
-        GG_CUDA(cudaStreamSynchronize(H.stream));
+        gg::copy_to_host(H, q, H.qtmp.p, sizeof(double) * H.nel);
     })
     return GG_OK;
 }
@@ -578,8 +567,7 @@ int gg_get_rhs(gg_handle* h, double* f, double* hvec) {
     GG_TRY2(h, {
         if (f) gg::nodal_out(H, H.f.as<double>(), f);
         if (hvec) {
-            GG_CUDA(cudaMemcpyAsync(hvec, H.hvec.p, sizeof(double) * H.nel, cudaMemcpyDeviceToHost, H.stream));
-            GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, hvec, H.hvec.p, sizeof(double) * H.nel);
         }
     })
     return GG_OK;
@@ -592,8 +580,7 @@ int gg_get_diagonals(gg_handle* h, double* k_diag, double* schur_diag) {
     GG_TRY2(h, {
         if (k_diag) gg::nodal_out(H, H.kdiag64.as<double>(), k_diag);
         if (schur_diag) {
-            GG_CUDA(cudaMemcpyAsync(schur_diag, H.sdiag.p, sizeof(double) * H.nel, cudaMemcpyDeviceToHost, H.stream));
-            GG_CUDA(cudaStreamSynchronize(H.stream));
+            gg::copy_to_host(H, schur_diag, H.sdiag.p, sizeof(double) * H.nel);
         }
     })
     return GG_OK;

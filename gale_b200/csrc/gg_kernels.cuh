@@ -9,6 +9,11 @@ namespace gg {
 
 int num_sms();
 int grid_for(int64_t n, int block);
+// Host arrays to and from the device (gg_copy.cu): complete on return / read on return.
+void copy_to_host(Handle& H, void* host, const void* device, size_t bytes);
+void copy_to_device(Handle& H, void* device, const void* host, size_t bytes);
+void copy_handle_created();
+void copy_handle_destroyed();
 // Record a message for gg_last_error and return the status code (gg_api.cu).
 int set_error(Handle& H, int code, const std::string& msg);
 

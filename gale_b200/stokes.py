@@ -310,17 +310,17 @@ class StokesProblem:
     def points(self):
         n = C.c_int64(0)
         self._check(self.lib.gg_point_count(self.h, C.byref(n)))
-        x = np.zeros((n.value, self.dim))
-        m = np.zeros(n.value, dtype=np.int32)
-        ps = np.zeros(n.value)
+        x = np.empty((n.value, self.dim))
+        m = np.empty(n.value, dtype=np.int32)
+        ps = np.empty(n.value)
         self._check(self.lib.gg_get_points(self.h, ptr(x), ptr(m, C.c_int32), ptr(ps)))
         return x, m, ps
 
     def integration_points(self):
         n = C.c_int64(0)
         self._check(self.lib.gg_point_count(self.h, C.byref(n)))
-        xi = np.zeros((n.value, self.dim))
-        w = np.zeros(n.value)
+        xi = np.empty((n.value, self.dim))
+        w = np.empty(n.value)
         self._check(self.lib.gg_get_integration_points(self.h, ptr(xi), ptr(w)))
         return xi, w
 
@@ -358,7 +358,8 @@ class StokesProblem:
         return u, p, st.as_dict()
 
     def advect(self, dt, u=None, order=2):
-        out = np.zeros((self.np, self.dim))
+        # written whole by the call; numpy backs large empty() arrays with huge pages, not zeros()
+        out = np.empty((self.np, self.dim))
         uu = f64(u)
         self._check(self.lib.gg_advect(self.h, dt, order, ptr(uu), ptr(out)))
         return out
@@ -443,7 +444,7 @@ class StokesProblem:
     def moments(self):
         n = C.c_int32(0)
         self._check(self.lib.gg_get_moments(self.h, None, C.byref(n)))
-        m = np.zeros((n.value, self.nel))
+        m = np.empty((n.value, self.nel))
         self._check(self.lib.gg_get_moments(self.h, ptr(m), None))
         return m
 
@@ -465,13 +466,13 @@ class StokesProblem:
         return q
 
     def rhs(self):
-        f = np.zeros(self.nnode * self.dim)
-        hv = np.zeros(self.nel)
+        f = np.empty(self.nnode * self.dim)
+        hv = np.empty(self.nel)
         self._check(self.lib.gg_get_rhs(self.h, ptr(f), ptr(hv)))
         return f, hv
 
     def diagonals(self):
-        kd = np.zeros(self.nnode * self.dim)
-        sd = np.zeros(self.nel)
+        kd = np.empty(self.nnode * self.dim)
+        sd = np.empty(self.nel)
         self._check(self.lib.gg_get_diagonals(self.h, ptr(kd), ptr(sd)))
         return kd, sd
