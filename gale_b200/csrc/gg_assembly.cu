@@ -16,17 +16,18 @@
 // points (sorted by element, in reference order) produces them; the K apply then never
 // touches a point again.
 //
-// Kernel shape: a CTA owns 128 consecutive elements and walks their contiguous point
-// range in chunks of 512.  Phase 1 (one thread per point, coalesced loads): rheology,
-// c_p, force weights → shared memory.  Phase 2 (one thread per element): sequential
-// sums in point order, i.e. the reference's summation order.  The element's corner terms
-// of the K diagonal and of the force go to per-element buffers; k_gather_corners sums
-// them per node in a fixed element order, so a build gives the same bits on every run.
-#include <map>
-#include <set>
-#include <condition_variable>
-#include <mutex>
-#include <tuple>
+// Two kernels.  k_points evaluates the rheology chain per point (one thread per point, both
+// precisions of a mixed build from the same loads) and leaves c_p and the force weights in
+// point order; k_moments sums them per element, four lanes per element, each lane its own
+// accumulators over the element's points in order -- the reference's summation order, and
+// the same bits whatever the launch shape.  As one kernel (rheology into shared memory, then
+// one thread per element with all 39 accumulators) the build held 255 registers, ran 8 warps
+// per SM at 0.9 instructions per cycle and took 752 µs (FP64) + 549 µs (FP32) for 7.1 M
+// points in 64³ elements; @@TIMES@@
+// The element's corner terms of the K diagonal and of the force go to per-element buffers;
+// k_gather_corners sums them per node in a fixed element order, so a build gives the same
+// bits on every run.
+#include <cmath>
 
 #include "gg_internal.cuh"
 #include "gg_kernels.cuh"
@@ -34,15 +35,6 @@
 namespace gg {
 
 namespace {
-
-// CTA shapes (elements per CTA = threads, points per shared-memory chunk) the autotuner
-// chooses from; the sums per element run in point order whatever the shape, so every
-// shape gives the same moments.
-struct BuildShape {
-    int epc, chunk;
-};
-constexpr BuildShape kShapes[] = {{64, 256}, {128, 256}, {128, 512}, {256, 512}};
-constexpr int kNumShapes = 4;
 
 template <typename R> __device__ __forceinline__ R r_exp(R x);
 template <> __device__ __forceinline__ double r_exp<double>(double x) { return exp(x); }
@@ -227,131 +219,140 @@ __device__ PointOut run_rheologies(const MeshK& mk, const gg_material& m, const 
     return out;
 }
 
-template <int DIM, typename R, int kElemPerCta, int kChunk>
-__global__ void __launch_bounds__(kElemPerCta)
-k_build_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets,
-                const double* __restrict__ xi_s, int64_t np_s, const int32_t* __restrict__ mat_s,
-                const double* __restrict__ ps_s, const double* __restrict__ T,
-                const double* __restrict__ pu, const double* __restrict__ pp, int prev,
-                double gravity, double g0, double g1, double g2, double rayleigh, int want_force,
-                R* __restrict__ mom, R* __restrict__ kcorner, double* __restrict__ sdiag,
-                double* __restrict__ fcorner, double* __restrict__ eta_s, double* __restrict__ incr_s,
-                uint8_t* __restrict__ yld_s, int32_t* __restrict__ flag,
-                const gg_material* __restrict__ materials, const double* __restrict__ w_s) {
-    constexpr int NM = n_moments<DIM>();
+// Per point: viscosity, its quadrature coefficient c_p = w_p detJ η_p (FP64, with kBoth also
+// FP32 from the FP32 rheology chain), the force weights φ_p = detJ w ρ g and
+// ψ_p = detJ w Ra T (null: zero for every point).  Bound by its loads and stores
+// (60-90 bytes per point) once enough warps cover the exponential's latency.
+template <int DIM, bool kBoth>
+__global__ void __launch_bounds__(256)
+k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const int32_t* __restrict__ offsets,
+         const double* __restrict__ xi_s, const int32_t* __restrict__ mat_s, const double* __restrict__ ps_s,
+         const double* __restrict__ w_s, const double* __restrict__ T, const double* __restrict__ pu,
+         const double* __restrict__ pp, int prev, double gravity, double rayleigh,
+         const gg_material* __restrict__ materials, double* __restrict__ c64, float* __restrict__ c32,
+         double* __restrict__ phi, double* __restrict__ psi, double* __restrict__ eta_s,
+         double* __restrict__ incr_s, uint8_t* __restrict__ yld_s) {
     constexpr int NEN = 1 << DIM;
-    __shared__ R s_c[kChunk];
-    __shared__ R s_xi[DIM][kChunk];
-    __shared__ double s_phi[kChunk];
-    __shared__ double s_psi[kChunk];
-
-    const int64_t e0 = (int64_t)blockIdx.x * kElemPerCta;
-    if (e0 >= nel) return;
-    const int64_t e1 = min(nel, e0 + kElemPerCta);
-    const int64_t e = e0 + threadIdx.x;
-    const bool own = e < e1;
-    const int32_t pbeg = offsets[e0], pend = offsets[e1];
-    const int32_t my_b = own ? offsets[e] : 0, my_e = own ? offsets[e + 1] : 0;
     const double wscale = (double)(1 << DIM);
-
-    R acc[NM];
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t pe = cell_s[i];
+        int ijk[3];
+        elem_ijk(mk, pe, ijk);
+        double xi[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int m = 0; m < NM; m++) acc[m] = R(0);
-    double F[NEN], Psi[NEN];
+        for (int d = 0; d < DIM; d++) xi[d] = xi_s[(int64_t)d * np + i];
+        const gg_material& m = materials[mat_s[i]];
+        const double ps = ps_s[i];
+        const PointOut po = run_rheologies<DIM, double>(mk, m, ijk, pe, xi, T, pu, pp, ps, prev);
+        // per-point weight (DVCWeights) or _ConstantWeights_Calculate
+        const double w = w_s ? w_s[i] : wscale / (double)(offsets[pe + 1] - offsets[pe]);
+        c64[i] = (w * mk.detJ) * po.eta;
+        eta_s[i] = po.eta;
+        incr_s[i] = po.incr;
+        yld_s[i] = po.yielded;
+        if (kBoth) {
+            float x32[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int a = 0; a < NEN; a++) { F[a] = 0.0; Psi[a] = 0.0; }
-
-    for (int32_t cs = pbeg; cs < pend; cs += kChunk) {
-        const int32_t ce = min(pend, cs + kChunk);
-        // ---- phase 1: one thread per point
-        for (int32_t i = cs + threadIdx.x; i < ce; i += blockDim.x) {
-            // element of sorted point i: binary search in this CTA's offsets
-            int lo = 0, hi = (int)(e1 - e0) - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (offsets[e0 + mid] <= i) lo = mid; else hi = mid - 1;
+            for (int d = 0; d < DIM; d++) x32[d] = (float)xi[d];
+            const PointOut pf = run_rheologies<DIM, float>(mk, m, ijk, pe, x32, T, pu, pp, ps, prev);
+            c32[i] = (float)(w * mk.detJ) * (float)pf.eta;
+        }
+        if (phi || psi) {
+            double Tp = 0.0;
+            if (T && (rayleigh != 0.0 || m.alpha != 0.0)) {
+                double N[NEN];
+                shape<DIM, double>(xi, N);
+#pragma unroll
+                for (int a = 0; a < NEN; a++) Tp += T[elem_node<DIM>(mk, ijk, a)] * N[a];
             }
-            const int64_t pe = e0 + lo;
-            int ijk[3];
-            elem_ijk(mk, pe, ijk);
-            R xi[3] = {R(0), R(0), R(0)};
-#pragma unroll
-            for (int d = 0; d < DIM; d++) xi[d] = (R)xi_s[(int64_t)d * np_s + i];
-            const int mi = mat_s[i];
-            const gg_material& m = materials[mi];
-            PointOut po = run_rheologies<DIM, R>(mk, m, ijk, pe, xi, T, pu, pp, ps_s[i], prev);
-            const int32_t cnt = offsets[pe + 1] - offsets[pe];
-            // per-point weight (DVCWeights) or _ConstantWeights_Calculate
-            const double w = w_s ? w_s[i] : wscale / (double)cnt;
-            s_c[i - cs] = (R)(w * mk.detJ) * (R)po.eta;
-#pragma unroll
-            for (int d = 0; d < DIM; d++) s_xi[d][i - cs] = xi[d];
-            if (want_force) {
-                double Tp = 0.0;
-                if (T && (rayleigh != 0.0 || m.alpha != 0.0)) {
-                    double xd[3] = {xi_s[i], xi_s[np_s + i], DIM == 3 ? xi_s[2 * np_s + i] : 0.0};
-                    double N[NEN];
-                    shape<DIM, double>(xd, N);
-#pragma unroll
-                    for (int a = 0; a < NEN; a++) Tp += T[elem_node<DIM>(mk, ijk, a)] * N[a];
-                }
+            if (phi) {
                 const double rho = m.density * (1.0 - m.alpha * Tp);
-                s_phi[i - cs] = mk.detJ * w * rho * gravity;
-                s_psi[i - cs] = mk.detJ * w * (rayleigh * Tp);
+                phi[i] = mk.detJ * w * rho * gravity;
             }
-            if (eta_s) {
-                eta_s[i] = po.eta;
-                incr_s[i] = po.incr;
-                yld_s[i] = po.yielded;
-            }
+            if (psi) psi[i] = mk.detJ * w * (rayleigh * Tp);
         }
-        __syncthreads();
-        // ---- phase 2: one thread per element, points in reference order
-        if (own) {
-            const int32_t b = max(my_b, cs), en = min(my_e, ce);
-            for (int32_t i = b; i < en; i++) {
-                const int k = i - cs;
-                const R c = s_c[k];
-                R px[3], py[3], pz[3];
-                px[0] = R(1); px[1] = s_xi[0][k]; px[2] = px[1] * px[1];
-                py[0] = R(1); py[1] = s_xi[1][k]; py[2] = py[1] * py[1];
-                pz[0] = R(1); pz[1] = DIM == 3 ? s_xi[DIM - 1][k] : R(0); pz[2] = pz[1] * pz[1];
-#pragma unroll
-                for (int cc = 0; cc < (DIM == 3 ? 3 : 1); cc++)
-#pragma unroll
-                    for (int bb = 0; bb < 3; bb++)
-#pragma unroll
-                        for (int aa = 0; aa < 3; aa++) {
-                            constexpr int dummy = 0;
-                            (void)dummy;
-                            const int slot = mom_slot<DIM>(aa, bb, cc);
-                            if (slot >= 0) acc[slot] += c * (px[aa] * py[bb] * pz[cc]);
-                        }
-                if (want_force) {
-                    double xd[3] = {(double)s_xi[0][k], (double)s_xi[1][k],
-                                    DIM == 3 ? (double)s_xi[DIM - 1][k] : 0.0};
-                    double N[NEN];
-                    shape<DIM, double>(xd, N);
-                    const double phi = s_phi[k], psi = s_psi[k];
-#pragma unroll
-                    for (int a = 0; a < NEN; a++) { F[a] += phi * N[a]; Psi[a] += psi * N[a]; }
-                }
-            }
-        }
-        __syncthreads();
     }
-    if (!own) return;
-    if (my_e == my_b) atomicAdd(flag, 1);  // empty element
-#pragma unroll
-    for (int m = 0; m < NM; m++) mom[(int64_t)m * nel + e] = acc[m];
+}
 
+// Per element, four lanes: lane q < 3 sums the moments of ξ-exponent q (every lane the same
+// instructions, with its own power of ξ), lane q the force terms of corners q·NC … (φ, ψ
+// null: none).  Then every lane takes all moments and forms its corners' diagonal terms.
+// Eight elements per warp keep an SM at 32 and more warps, where one thread per element and
+// 39 accumulators left 8; the eight streams of points of a warp meet in L1.
+template <int DIM, typename R, bool kForce>
+__global__ void __launch_bounds__(128)
+k_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets, const double* __restrict__ xi_s, int64_t np,
+          const R* __restrict__ cp, const double* __restrict__ phi, const double* __restrict__ psi,
+          R* __restrict__ mom, R* __restrict__ kcorner, double* __restrict__ sdiag, double* __restrict__ fcorner,
+          int32_t* __restrict__ flag) {
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr int NM = n_moments<DIM>(), NEN = 1 << DIM, NC = NEN / 4, NZ = DIM == 3 ? 3 : 1;
+    const int q = threadIdx.x & 3;
+    const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const bool own = e < nel;
+    const int32_t b = own ? offsets[e] : 0, en = own ? offsets[e + 1] : 0;
+    R acc[3][NZ];
+#pragma unroll
+    for (int bb = 0; bb < 3; bb++)
+#pragma unroll
+        for (int cc = 0; cc < NZ; cc++) acc[bb][cc] = R(0);
+    double F[NC], Psi[NC];
+#pragma unroll
+    for (int j = 0; j < NC; j++) { F[j] = 0.0; Psi[j] = 0.0; }
+#pragma unroll 4
+    for (int32_t i = b; i < en; i++) {
+        const double xd = xi_s[i], yd = xi_s[np + i], zd = DIM == 3 ? xi_s[2 * np + i] : 0.0;
+        const R c = cp[i], x = (R)xd, y = (R)yd, z = (R)zd;
+        const R px = q == 0 ? R(1) : q == 1 ? x : x * x;
+        const R pxy[3] = {px, px * y, px * (y * y)};
+        const R zz = z * z;
+#pragma unroll
+        for (int bb = 0; bb < 3; bb++) {
+            acc[bb][0] += c * pxy[bb];
+            if (DIM == 3) {
+                acc[bb][NZ == 3 ? 1 : 0] += c * (pxy[bb] * z);
+                acc[bb][NZ == 3 ? 2 : 0] += c * (pxy[bb] * zz);
+            }
+        }
+        if (kForce) {
+            const double ph = phi ? phi[i] : 0.0, ps = psi ? psi[i] : 0.0;
+#pragma unroll
+            for (int j = 0; j < NC; j++) {
+                const int a = q * NC + j;
+                double N = DIM == 2 ? 0.25 : 0.125;
+                N *= 1.0 + ((a & 1) ? xd : -xd);
+                N *= 1.0 + ((a & 2) ? yd : -yd);
+                if (DIM == 3) N *= 1.0 + ((a & 4) ? zd : -zd);
+                F[j] += ph * N;
+                Psi[j] += ps * N;
+            }
+        }
+    }
+    if (own && q == 0 && en == b) atomicAdd(flag, 1);  // empty element
+    R M[NM];
+#pragma unroll
+    for (int aa = 0; aa < 3; aa++)
+#pragma unroll
+        for (int bb = 0; bb < 3; bb++)
+#pragma unroll
+            for (int cc = 0; cc < NZ; cc++) {
+                const int slot = mom_slot<DIM>(aa, bb, cc);
+                if (slot >= 0) M[slot] = __shfl_sync(kFull, acc[bb][cc], aa, 4);
+            }
+    if (own) {
+#pragma unroll
+        for (int m = 0; m < NM; m++)
+            if ((m & 3) == q) mom[(int64_t)m * nel + e] = M[m];
+    }
     // element diagonal of K from the moments:
     // K[(a,c),(a,c)] = Σ_p c_p [ Σ_d (∂N_a/∂x_d)² + (∂N_a/∂x_c)² ]
-    int ijk[3];
-    elem_ijk(mk, e, ijk);
-    double sd = 0.0;
+    double ratio[NC][DIM], G[NC][DIM];  // G_e / K_e diagonal and G_e of this lane's dofs
 #pragma unroll
-    for (int a = 0; a < NEN; a++) {
+    for (int j = 0; j < NC; j++) {
+        const int a = q * NC + j;
+        double sg[3];
+#pragma unroll
+        for (int o = 0; o < 3; o++) sg[o] = ((a >> o) & 1) ? 1.0 : -1.0;
         double S[3];
 #pragma unroll
         for (int d = 0; d < DIM; d++) {
@@ -363,18 +364,16 @@ k_build_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets,
                 for (int k1 = 0; k1 < 3; k1++)
 #pragma unroll
                     for (int k2 = 0; k2 < 3; k2++) {
-                        int ex[3] = {k0, k1, k2};
+                        const int ex[3] = {k0, k1, k2};
                         bool ok = true;
                         double coef = 1.0;
 #pragma unroll
                         for (int o = 0; o < 3; o++) {
                             if (o >= DIM || o == d) { if (ex[o] != 0) ok = false; continue; }
-                            const double s = ((a >> o) & 1) ? 1.0 : -1.0;
-                            coef *= ex[o] == 1 ? 2.0 * s : 1.0;
+                            coef *= ex[o] == 1 ? 2.0 * sg[o] : 1.0;
                         }
                         if (!ok) continue;
-                        const int slot = mom_slot<DIM>(k0, k1, k2);
-                        v += coef * (double)acc[slot];
+                        v += coef * (double)M[mom_slot<DIM>(k0, k1, k2)];
                     }
             S[d] = v * mk.kappa[d] * mk.kappa[d];
         }
@@ -384,16 +383,32 @@ k_build_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets,
 #pragma unroll
         for (int c = 0; c < DIM; c++) {
             const double dg = tot + S[c];
-            kcorner[(int64_t)(a * DIM + c) * nel + e] = (R)dg;
-            // Ĝ_e = Σ G_e² / K_e diagonal, over every dof (UzawaPreconditionerTerm.cxx:199-215)
-            sd += mk.Ge[a][c] * (mk.Ge[a][c] / dg);
+            if (own) kcorner[(int64_t)(a * DIM + c) * nel + e] = (R)dg;
+            if (kForce) {
+                G[j][c] = mk.Ge[a][c];
+                ratio[j][c] = G[j][c] / dg;
+            }
         }
-        if (want_force) {
-            fcorner[(int64_t)a * nel + e] = F[a];
-            fcorner[(int64_t)(NEN + a) * nel + e] = Psi[a];
+        if (kForce && own) {
+            fcorner[(int64_t)a * nel + e] = F[j];
+            fcorner[(int64_t)(NEN + a) * nel + e] = Psi[j];
         }
     }
-    if (sdiag) sdiag[e] = sd;
+    if (kForce) {
+        // Ĝ_e = Σ G_e² / K_e diagonal, over every dof (UzawaPreconditionerTerm.cxx:199-215), in
+        // dof order: the running sum passes from lane to lane
+        double sd = 0.0;
+#pragma unroll
+        for (int l = 0; l < 4; l++) {
+            double s = sd;
+#pragma unroll
+            for (int j = 0; j < NC; j++)
+#pragma unroll
+                for (int c = 0; c < DIM; c++) s += G[j][c] * ratio[j][c];
+            sd = __shfl_sync(kFull, s, l, 4);
+        }
+        if (own && q == 0) sdiag[e] = sd;
+    }
 }
 
 // Node sums of the element corner terms in a fixed element order (corner a' = 0 … 2^dim−1
@@ -449,23 +464,6 @@ void upload_materials(Handle& H) {
                             cudaMemcpyHostToDevice, H.stream));
 }
 
-template <int DIM, typename R, int EPC, int CH>
-static void launch_shape(Handle& H, int prev, const double* pu, const double* pp, R* mom, R* kdiag, double* sdiag,
-                         double* f, bool outputs) {
-    const int64_t nel = H.nel;
-    const int grid = (int)((nel + EPC - 1) / EPC);
-    const double* T = H.has_T ? H.T.as<double>() : nullptr;
-    double g[3] = {H.force.g_hat[0], H.force.g_hat[1], H.force.g_hat[2]};
-    k_build_moments<DIM, R, EPC, CH><<<grid, EPC, 0, H.stream>>>(
-        H.mk, nel, H.offsets.as<int32_t>(), H.xi_s.as<double>(), H.np_in, H.mat_s.as<int32_t>(),
-        H.ps_s.as<double>(), T, pu, pp, prev, H.force.gravity, g[0], g[1], g[2], H.force.rayleigh,
-        f ? 1 : 0, mom, reinterpret_cast<R*>(H.kcorner.p), sdiag, f ? H.fcorner.as<double>() : nullptr,
-        outputs ? H.eta_s.as<double>() : nullptr,
-        H.incr_s.as<double>(), H.yld_s.as<uint8_t>(), H.flag.as<int32_t>(), H.d_materials.as<gg_material>(),
-        H.weights.mode == GG_WEIGHTS_DVC && H.dvc_valid ? H.w_s.as<double>() : nullptr);
-    GG_CUDA(cudaGetLastError());
-}
-
 // kdiag (and f) from the corner terms of the last build launch
 template <int DIM, typename R>
 static void gather_corners(Handle& H, R* kdiag, double* f) {
@@ -476,95 +474,54 @@ static void gather_corners(Handle& H, R* kdiag, double* f) {
     GG_CUDA(cudaGetLastError());
 }
 
-template <int DIM, typename R>
-static void launch_build_shape(int shape, Handle& H, int prev, const double* pu, const double* pp, R* mom, R* kdiag,
-                               double* sdiag, double* f, bool outputs) {
-    switch (shape) {
-        case 0: launch_shape<DIM, R, 64, 256>(H, prev, pu, pp, mom, kdiag, sdiag, f, outputs); break;
-        case 1: launch_shape<DIM, R, 128, 256>(H, prev, pu, pp, mom, kdiag, sdiag, f, outputs); break;
-        case 2: launch_shape<DIM, R, 128, 512>(H, prev, pu, pp, mom, kdiag, sdiag, f, outputs); break;
-        default: launch_shape<DIM, R, 256, 512>(H, prev, pu, pp, mom, kdiag, sdiag, f, outputs); break;
-    }
+// Whether the force weights of a build can be anything but zero: a zero gravity or Rayleigh
+// number makes them zero unless a factor beside it is not finite (a density, or through a
+// thermal expansivity the temperature).
+static bool any_alpha(const Handle& H) {
+    for (const gg_material& m : H.materials)
+        if (H.has_T && m.alpha != 0.0) return true;
+    return false;
 }
-
-// Autotuner: the first build of a (device, dim, precision, points-per-element class) times
-// every CTA shape twice on the real inputs (each trial overwrites every output) and keeps
-// the fastest for the rest of the process.  One thread tunes a key while the builds of
-// other threads with the same key wait for its choice: concurrent tunings would time each
-// other's launches and pick a shape at random.
-struct BuildTuner {
-    std::mutex mu;
-    std::condition_variable cv;
-    std::map<std::tuple<int, int, int, int>, int> best;
-    std::set<std::tuple<int, int, int, int>> busy;
-};
-static BuildTuner& tuner() {
-    static BuildTuner t;
-    return t;
+static bool phi_nonzero(const Handle& H) {
+    if (H.force.gravity != 0.0 || any_alpha(H)) return true;
+    for (const gg_material& m : H.materials)
+        if (!std::isfinite(m.density)) return true;
+    return false;
 }
+static bool psi_nonzero(const Handle& H) { return H.has_T && (H.force.rayleigh != 0.0 || any_alpha(H)); }
 
-template <int DIM, typename R>
-static void launch_build(Handle& H, int prev, const double* pu, const double* pp, R* mom, R* kdiag,
-                         double* sdiag, double* f, bool outputs) {
-    int dev = 0;
-    GG_CUDA(cudaGetDevice(&dev));
-    const double ppe = H.nel ? (double)H.np_in / (double)H.nel : 0.0;
-    const int klass = ppe < 12 ? 0 : ppe < 24 ? 1 : ppe < 48 ? 2 : 3;
-    const auto key = std::make_tuple(dev, DIM, (int)sizeof(R), klass);
-    int shape = -1;
-    bool tune = false;
-    {
-        std::unique_lock<std::mutex> lk(tuner().mu);
-        for (;;) {
-            auto it = tuner().best.find(key);
-            if (it != tuner().best.end()) {
-                shape = it->second;
-                break;
-            }
-            if (!tuner().busy.count(key)) {
-                tuner().busy.insert(key);
-                tune = true;
-                break;
-            }
-            tuner().cv.wait(lk);
-        }
+template <int DIM>
+static void launch_build(Handle& H, bool mixed, int prev, const double* pu, const double* pp) {
+    const int64_t np = H.np_in, nel = H.nel;
+    cudaStream_t st = H.stream;
+    const double* T = H.has_T ? H.T.as<double>() : nullptr;
+    const double* w = H.weights.mode == GG_WEIGHTS_DVC && H.dvc_valid ? H.w_s.as<double>() : nullptr;
+    double* phi = phi_nonzero(H) ? H.pt_phi.as<double>() : nullptr;
+    double* psi = psi_nonzero(H) ? H.pt_psi.as<double>() : nullptr;
+    double* c64 = H.pt_c64.as<double>();
+    float* c32 = mixed ? H.pt_c32.as<float>() : nullptr;
+    auto points = [&](auto kernel) {
+        kernel<<<grid_for(np, 256), 256, 0, st>>>(
+            H.mk, np, H.cell_s.as<int32_t>(), H.offsets.as<int32_t>(), H.xi_s.as<double>(), H.mat_s.as<int32_t>(),
+            H.ps_s.as<double>(), w, T, pu, pp, prev, H.force.gravity, H.force.rayleigh, H.d_materials.as<gg_material>(),
+            c64, c32, phi, psi, H.eta_s.as<double>(), H.incr_s.as<double>(), H.yld_s.as<uint8_t>());
+        GG_CUDA(cudaGetLastError());
+    };
+    if (mixed) points(k_points<DIM, true>);
+    else points(k_points<DIM, false>);
+    const unsigned grid = (unsigned)((4 * nel + 127) / 128);
+    k_moments<DIM, double, true><<<grid, 128, 0, st>>>(
+        H.mk, nel, H.offsets.as<int32_t>(), H.xi_s.as<double>(), np, c64, phi, psi, H.mom64.as<double>(),
+        H.kcorner.as<double>(), H.sdiag.as<double>(), H.fcorner.as<double>(), H.flag.as<int32_t>());
+    GG_CUDA(cudaGetLastError());
+    gather_corners<DIM, double>(H, H.kdiag64.as<double>(), H.f.as<double>());
+    if (mixed) {
+        k_moments<DIM, float, false><<<grid, 128, 0, st>>>(
+            H.mk, nel, H.offsets.as<int32_t>(), H.xi_s.as<double>(), np, c32, nullptr, nullptr, H.mom32.as<float>(),
+            H.kcorner.as<float>(), nullptr, nullptr, H.flag.as<int32_t>());
+        GG_CUDA(cudaGetLastError());
+        gather_corners<DIM, float>(H, H.kdiag32.as<float>(), nullptr);
     }
-    if (tune) {
-        float best_ms = 1e30f;
-        int best = 2;
-        try {
-            for (int rep = 0; rep < 2; rep++)
-                for (int k = 0; k < kNumShapes; k++) {
-                    GG_CUDA(cudaEventRecord(H.ev0, H.stream));
-                    launch_build_shape<DIM, R>(k, H, prev, pu, pp, mom, kdiag, sdiag, f, outputs);
-                    GG_CUDA(cudaEventRecord(H.ev1, H.stream));
-                    GG_CUDA(cudaEventSynchronize(H.ev1));
-                    float ms = 0.f;
-                    GG_CUDA(cudaEventElapsedTime(&ms, H.ev0, H.ev1));
-                    if (ms < best_ms) {
-                        best_ms = ms;
-                        best = k;
-                    }
-                }
-        } catch (...) {
-            {
-                std::lock_guard<std::mutex> lk(tuner().mu);
-                tuner().busy.erase(key);
-            }
-            tuner().cv.notify_all();
-            throw;
-        }
-        shape = best;
-        {
-            std::lock_guard<std::mutex> lk(tuner().mu);
-            tuner().best[key] = shape;
-            tuner().busy.erase(key);
-        }
-        tuner().cv.notify_all();
-    }
-    H.build_shape[sizeof(R) == 4 ? 1 : 0] = shape;
-    launch_build_shape<DIM, R>(shape, H, prev, pu, pp, mom, kdiag, sdiag, f, outputs);
-    gather_corners<DIM, R>(H, kdiag, f);
 }
 
 int build_operator(Handle& H, int precision, int prev, const double* d_prev_u,
@@ -583,22 +540,17 @@ int build_operator(Handle& H, int precision, int prev, const double* d_prev_u,
     H.fcorner.ensure(sizeof(double) * 2 * nen * nel);
     upload_materials(H);
     GG_CUDA(cudaMemsetAsync(H.flag.p, 0, sizeof(int32_t) * 4, st));
-    if (H.dim == 2)
-        launch_build<2, double>(H, prev, d_prev_u, d_prev_p, H.mom64.as<double>(), H.kdiag64.as<double>(),
-                                H.sdiag.as<double>(), H.f.as<double>(), true);
-    else
-        launch_build<3, double>(H, prev, d_prev_u, d_prev_p, H.mom64.as<double>(), H.kdiag64.as<double>(),
-                                H.sdiag.as<double>(), H.f.as<double>(), true);
-    if (precision == GG_PRECISION_MIXED) {
+    const bool mixed = precision == GG_PRECISION_MIXED;
+    H.pt_c64.ensure(sizeof(double) * H.np_in);
+    if (phi_nonzero(H)) H.pt_phi.ensure(sizeof(double) * H.np_in);
+    if (psi_nonzero(H)) H.pt_psi.ensure(sizeof(double) * H.np_in);
+    if (mixed) {
+        H.pt_c32.ensure(sizeof(float) * H.np_in);
         H.mom32.ensure(sizeof(float) * nm * nel);
         H.kdiag32.ensure(sizeof(float) * nd);
-        if (H.dim == 2)
-            launch_build<2, float>(H, prev, d_prev_u, d_prev_p, H.mom32.as<float>(), H.kdiag32.as<float>(),
-                                   nullptr, nullptr, false);
-        else
-            launch_build<3, float>(H, prev, d_prev_u, d_prev_p, H.mom32.as<float>(), H.kdiag32.as<float>(),
-                                   nullptr, nullptr, false);
     }
+    if (H.dim == 2) launch_build<2>(H, mixed, prev, d_prev_u, d_prev_p);
+    else launch_build<3>(H, mixed, prev, d_prev_u, d_prev_p);
     int32_t empty = 0;
     GG_CUDA(cudaMemcpyAsync(&empty, H.flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));

@@ -98,6 +98,7 @@ struct Handle {
 
     // operator
     DBuf mom64, mom32, kdiag64, kdiag32, sdiag, hvec, f;
+    DBuf pt_c64, pt_c32, pt_phi, pt_psi;  // per-point quadrature and force weights (build scratch)
     DBuf kcorner, fcorner;  // per-element corner terms of the diagonal / force (build scratch)
     bool built = false;
     int built_precision = -1;
@@ -119,7 +120,6 @@ struct Handle {
     int64_t coarse_n = 0;   // 0: no dense coarse solve (Chebyshev on the coarsest level)
     int64_t coarse_ld = 0;  // row stride of coarse_inv (coarse_n rounded up to 4)
     int mg_degree = 2;      // Chebyshev degree of the smoother
-    int build_shape[2] = {-1, -1};  // autotuned CTA shape of the FP64 / FP32 moment build
     // persistent multigrid FCG (gg_fused.cu): level table for the current hierarchy
     DBuf fused_tab, fused_part, fused_bar, fused_out;
     std::vector<unsigned char> fused_host;
