@@ -16,7 +16,8 @@ namespace gg {
 namespace {
 
 template <int DIM>
-__device__ bool velocity_at(const MeshK& mk, const double* x, const double* __restrict__ u, double* v) {
+__device__ bool velocity_at(const MeshK& mk, const double* x, const double2* __restrict__ axes,
+                            const double2* __restrict__ u, double* v) {
     int inds[3] = {0, 0, 0};
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
@@ -36,21 +37,29 @@ __device__ bool velocity_at(const MeshK& mk, const double* x, const double* __re
         }
     }
     double xi[3] = {0, 0, 0};
+    const double2* ax = axes;
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
-        const double lo = vert_coord_d(mk, d, inds[d]), hi = vert_coord_d(mk, d, inds[d] + 1);
-        xi[d] = __ddiv_rn(__dsub_rn(x[d], __dmul_rn(0.5, __dadd_rn(lo, hi))), __dmul_rn(0.5, __dsub_rn(hi, lo)));
+        const double2 g = ax[inds[d]];
+        xi[d] = __ddiv_rn(__dsub_rn(x[d], g.x), g.y);
+        ax += mk.n[d];
     }
 #pragma unroll
     for (int c = 0; c < DIM; c++) v[c] = 0.0;
+    const int32_t n0 = inds[0] + mk.nn[0] * (inds[1] + (DIM == 3 ? mk.nn[1] * inds[2] : 0));
 #pragma unroll
     for (int a = 0; a < (1 << DIM); a++) {
         double N = (DIM == 2) ? 0.25 : 0.125;
 #pragma unroll
         for (int d = 0; d < DIM; d++) N *= 1.0 + (((a >> d) & 1) ? xi[d] : -xi[d]);
-        const int64_t n = elem_node<DIM>(mk, inds, a);
+        const int32_t n = n0 + (a & 1) + ((a >> 1) & 1) * mk.nn[0] + (DIM == 3 ? ((a >> 2) & 1) * mk.nn[0] * mk.nn[1] : 0);
+        double uc[4];
+        const double2 u01 = u[(int64_t)n * (DIM - 1)];
+        uc[0] = u01.x;
+        uc[1] = u01.y;
+        if (DIM == 3) uc[2] = u[(int64_t)n * (DIM - 1) + 1].x;
 #pragma unroll
-        for (int c = 0; c < DIM; c++) v[c] += u[(int64_t)c * mk.nnode + n] * N;
+        for (int c = 0; c < DIM; c++) v[c] += uc[c] * N;
     }
 #pragma unroll
     for (int c = 0; c < DIM; c++)
@@ -58,16 +67,29 @@ __device__ bool velocity_at(const MeshK& mk, const double* x, const double* __re
     return true;
 }
 
+// velocity per node, [nnode][2] or [nnode][4], from the component-major vector
 template <int DIM>
-__global__ void k_advect(MeshK mk, int64_t np, double dt, int order, const double* __restrict__ u,
-                         double* __restrict__ coords, int32_t* __restrict__ flag) {
+__global__ void k_node_velocity(int64_t nnode, const double* __restrict__ u, double2* __restrict__ out) {
+    for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nnode; n += (int64_t)gridDim.x * blockDim.x) {
+        out[n * (DIM - 1)] = make_double2(u[n], u[nnode + n]);
+        if (DIM == 3) out[n * 2 + 1] = make_double2(u[2 * nnode + n], 0.0);
+    }
+}
+
+// Bound by the corner velocities: the points are in no spatial order, so every corner is a
+// sector of its own.  With the components in separate vectors a 3D stage read 24 of them per
+// point; a node's components in one 32-byte sector make it 8 (7.1 M points, two stages:
+// 978 → 639 µs).
+template <int DIM>
+__global__ void k_advect(MeshK mk, int64_t np, double dt, int order, const double2* __restrict__ axes,
+                         const double2* __restrict__ u, double* __restrict__ coords, int32_t* __restrict__ flag) {
     const double hdt = __dmul_rn(0.5, dt);
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
          p += (int64_t)gridDim.x * blockDim.x) {
         double x0[3], x[3], k1[3], k2[3];
 #pragma unroll
         for (int c = 0; c < DIM; c++) x0[c] = coords[p * DIM + c];
-        if (!velocity_at<DIM>(mk, x0, u, k1)) {
+        if (!velocity_at<DIM>(mk, x0, axes, u, k1)) {
             atomicAdd(flag, 1);
             continue;
         }
@@ -77,7 +99,7 @@ __global__ void k_advect(MeshK mk, int64_t np, double dt, int order, const doubl
         } else {
 #pragma unroll
             for (int c = 0; c < DIM; c++) x[c] = __dadd_rn(x0[c], __dmul_rn(hdt, k1[c]));
-            if (velocity_at<DIM>(mk, x, u, k2)) {
+            if (velocity_at<DIM>(mk, x, axes, u, k2)) {
 #pragma unroll
                 for (int c = 0; c < DIM; c++) x[c] = __dadd_rn(x0[c], __dmul_rn(dt, k2[c]));
             } else {
@@ -97,10 +119,17 @@ int advect(Handle& H, double dt, int order, const double* d_u, double* d_out) {
     H.flag.ensure(sizeof(int32_t) * 4);
     GG_CUDA(cudaMemsetAsync(H.flag.p, 0, sizeof(int32_t) * 4, H.stream));
     const int g = grid_for(H.np, 256);
-    if (H.dim == 2)
-        k_advect<2><<<g, 256, 0, H.stream>>>(H.mk, H.np, dt, order, d_u, H.coords.as<double>(), H.flag.as<int32_t>());
-    else
-        k_advect<3><<<g, 256, 0, H.stream>>>(H.mk, H.np, dt, order, d_u, H.coords.as<double>(), H.flag.as<int32_t>());
+    const double2* axes = element_axes(H);
+    H.adv_u.ensure(sizeof(double2) * H.nnode * (H.dim - 1));
+    double2* un = H.adv_u.as<double2>();
+    const int gn = grid_for(H.nnode, 256);
+    if (H.dim == 2) {
+        k_node_velocity<2><<<gn, 256, 0, H.stream>>>(H.nnode, d_u, un);
+        k_advect<2><<<g, 256, 0, H.stream>>>(H.mk, H.np, dt, order, axes, un, H.coords.as<double>(), H.flag.as<int32_t>());
+    } else {
+        k_node_velocity<3><<<gn, 256, 0, H.stream>>>(H.nnode, d_u, un);
+        k_advect<3><<<g, 256, 0, H.stream>>>(H.mk, H.np, dt, order, axes, un, H.coords.as<double>(), H.flag.as<int32_t>());
+    }
     GG_CUDA(cudaGetLastError());
     int32_t bad = 0;
     GG_CUDA(cudaMemcpyAsync(&bad, H.flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, H.stream));

@@ -312,6 +312,7 @@ int gg_set_points(gg_handle* h, int64_t n, const double* coords, const int32_t* 
     GG_TRY(h, {
         const int dim = H.dim;
         H.np = n;
+        H.ps_given = plastic_strain != nullptr;
         H.coords.ensure(sizeof(double) * n * dim);
         H.mat_in.ensure(sizeof(int32_t) * n);
         H.ps_in.ensure(sizeof(double) * n);

@@ -23,7 +23,8 @@
 // the same bits whatever the launch shape.  As one kernel (rheology into shared memory, then
 // one thread per element with all 39 accumulators) the build held 255 registers, ran 8 warps
 // per SM at 0.9 instructions per cycle and took 752 µs (FP64) + 549 µs (FP32) for 7.1 M
-// points in 64³ elements; @@TIMES@@
+// points in 64³ elements; now k_points takes 280 µs for both precisions, k_moments 166 µs
+// (FP64) and 108 µs (FP32).
 // The element's corner terms of the K diagonal and of the force go to per-element buffers;
 // k_gather_corners sums them per node in a fixed element order, so a build gives the same
 // bits on every run.
@@ -222,9 +223,11 @@ __device__ PointOut run_rheologies(const MeshK& mk, const gg_material& m, const 
 // Per point: viscosity, its quadrature coefficient c_p = w_p detJ η_p (FP64, with kBoth also
 // FP32 from the FP32 rheology chain), the force weights φ_p = detJ w ρ g and
 // ψ_p = detJ w Ra T (null: zero for every point).  Bound by its loads and stores
-// (60-90 bytes per point) once enough warps cover the exponential's latency.
+// (60-90 bytes per point) once enough warps cover the exponential's latency: at 255
+// registers, one block per SM, it took 651 µs for 7.1 M points; three blocks spill a little
+// in the yield laws and take 280 (two: 290), 32-bit element indices in both.
 template <int DIM, bool kBoth>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
 k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const int32_t* __restrict__ offsets,
          const double* __restrict__ xi_s, const int32_t* __restrict__ mat_s, const double* __restrict__ ps_s,
          const double* __restrict__ w_s, const double* __restrict__ T, const double* __restrict__ pu,
@@ -235,9 +238,9 @@ k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const int32_t
     constexpr int NEN = 1 << DIM;
     const double wscale = (double)(1 << DIM);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pe = cell_s[i];
-        int ijk[3];
-        elem_ijk(mk, pe, ijk);
+        const uint32_t pe = (uint32_t)cell_s[i], row = pe / (uint32_t)mk.n[0];
+        const int ijk[3] = {(int)(pe - row * (uint32_t)mk.n[0]), (int)(row % (uint32_t)mk.n[1]),
+                            (int)(row / (uint32_t)mk.n[1])};
         double xi[3] = {0.0, 0.0, 0.0};
 #pragma unroll
         for (int d = 0; d < DIM; d++) xi[d] = xi_s[(int64_t)d * np + i];

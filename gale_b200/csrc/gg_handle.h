@@ -85,6 +85,9 @@ struct Handle {
     int64_t np = 0, np_in = 0;
     DBuf coords, mat_in, ps_in, cell, perm, cell_s, xi_s, mat_s, ps_s, eta_s, incr_s, yld_s;
     DBuf offsets, fill, scan_tmp, flag;
+    DBuf axes;               // centre and half width of every element per axis
+    bool ps_given = false;   // a plastic strain was passed with the points (else it is zero)
+    DBuf adv_u;              // velocity per node, padded to whole words of 16 or 32 bytes
     bool located = false;
     // integration weights (gg_dvc.cu): with GG_WEIGHTS_DVC, xi_s holds the Voronoi
     // centroids and w_s the volumes of the sorted points once dvc_valid; xi_pts keeps

@@ -14,6 +14,16 @@ void copy_to_host(Handle& H, void* host, const void* device, size_t bytes);
 void copy_to_device(Handle& H, void* device, const void* host, size_t bytes);
 void copy_handle_created();
 void copy_handle_destroyed();
+// Point sort (gg_points.cu): an element below 2^kCellBits and the point's place in it, up to
+// kPlaceMax, share a word; elements of up to kPlaceSort points are sorted in place.
+constexpr int kCellBits = 21;
+constexpr int kPlaceMax = (1 << (32 - kCellBits)) - 1;
+constexpr int kPlaceSort = 1024;
+constexpr int kSegBlock = 128;                          // elements (and threads) per block of the sort
+constexpr int kSegCap = (kSegBlock / 32) * 1280;        // point indices of a block in shared memory
+static_assert(kSegCap >= (kSegBlock / 32) * kPlaceSort, "a warp's share holds the largest element");
+// centre and half width of every element per axis (built on first use)
+const double2* element_axes(Handle& H);
 // Record a message for gg_last_error and return the status code (gg_api.cu).
 int set_error(Handle& H, int code, const std::string& msg);
 

@@ -31,20 +31,25 @@ MeshK make_mesh(const gg_mesh_desc& d);
 
 // kernels of gg_points.cu (same arithmetic as gg_locate)
 __global__ void k_locate(MeshK mk, int64_t np, const double* __restrict__ x, uint32_t* __restrict__ cell,
-                         int32_t* __restrict__ count, int32_t* __restrict__ flag);
+                         int32_t* __restrict__ count, int32_t* __restrict__ flag, int32_t* __restrict__ place);
 __global__ void k_scan_blocks(const int32_t* __restrict__ in, int64_t n, int32_t* __restrict__ out,
                               int32_t* __restrict__ block_sums);
 __global__ void k_scan_sums(int32_t* __restrict__ sums, int64_t nblocks, int32_t* __restrict__ total);
 __global__ void k_scan_add(int32_t* __restrict__ out, int64_t n, const int32_t* __restrict__ sums,
                            const int32_t* __restrict__ total);
-__global__ void k_scatter(int64_t np, int64_t nel, const uint32_t* __restrict__ cell,
-                          const int32_t* __restrict__ offsets, int32_t* __restrict__ fill,
-                          int32_t* __restrict__ unsorted);
+void launch_scatter(int64_t np, int64_t nel, uint32_t* cell, const int32_t* offsets, const int32_t* place,
+                    int32_t* unsorted, cudaStream_t st);
+template <bool kInPlace>
+__global__ void k_segsort(int64_t nel, const int32_t* __restrict__ offsets, int32_t* unsorted, int32_t* perm,
+                          int32_t* flags);
+int segsort_grid(int64_t nel);
 
 namespace {
 
 constexpr int64_t kNoAllocMaxElements = 1 << 20;  // 1,048,576 elements
-constexpr int kNoAllocMaxPerElement = 1024;       // points per element
+constexpr int kNoAllocMaxPerElement = kPlaceSort; // points per element
+static_assert(kNoAllocMaxElements < (int64_t(1) << kCellBits), "an element and its point's place share a word");
+static_assert(kNoAllocMaxPerElement <= kPlaceMax, "places of a legal element fit their bits");
 constexpr int64_t kScanBlocks = (kNoAllocMaxElements + 1023) / 1024;
 // layout: [counts: max+1][block sums: kScanBlocks+2][flags: 4]
 constexpr int64_t kCountsOff = 0;
@@ -57,34 +62,6 @@ __device__ __align__(256) int32_t g_noalloc_scratch[kScratchWords];
 
 int32_t* g_scratch_addr[kMaxDevices] = {nullptr};
 std::mutex g_scratch_mutex;
-
-// One warp per element: sort the element's point indices ascending, in place, through a
-// per-warp shared-memory copy (the point indices are distinct).  Flags an element that
-// holds more than kNoAllocMaxPerElement points.
-__global__ void k_segsort_inplace(int64_t nel, const int32_t* __restrict__ offsets, int32_t* __restrict__ order,
-                                  int32_t* __restrict__ flags) {
-    constexpr int kWarps = 4;
-    __shared__ int32_t seg[kWarps][kNoAllocMaxPerElement];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t e = warp; e < nel; e += nwarps) {
-        const int32_t b = offsets[e], n = offsets[e + 1] - b;
-        if (n > kNoAllocMaxPerElement) {
-            if (lane == 0) atomicAdd(&flags[1], 1);
-            continue;
-        }
-        for (int k = lane; k < n; k += 32) seg[wib][k] = order[b + k];
-        __syncwarp();
-        for (int k = lane; k < n; k += 32) {
-            const int32_t v = seg[wib][k];
-            int rank = 0;
-            for (int j = 0; j < n; j++) rank += (seg[wib][j] < v);
-            order[b + rank] = v;
-        }
-        __syncwarp();
-    }
-}
 
 int grid_of(int64_t n, int block) {
     int64_t g = (n + block - 1) / block;
@@ -173,7 +150,7 @@ extern "C" GG_API int gg_locate_noalloc(const gg_mesh_desc* mesh, int64_t n_poin
         *msg = what;
         return false;
     };
-    k_locate<<<grid_of(n_points, 256), 256, 0, st>>>(mk, n_points, d_coords, d_cell, counts, flags);
+    k_locate<<<grid_of(n_points, 256), 256, 0, st>>>(mk, n_points, d_coords, d_cell, counts, flags, nullptr);
     if (!launched("gg_locate_noalloc: launch of the location kernel failed")) return GG_ERR_CUDA;
     k_scan_blocks<<<(int)nblk, 1024, 0, st>>>(counts, nel, d_offsets, sums);
     if (!launched("gg_locate_noalloc: launch of the block scan failed")) return GG_ERR_CUDA;
@@ -181,13 +158,10 @@ extern "C" GG_API int gg_locate_noalloc(const gg_mesh_desc* mesh, int64_t n_poin
     if (!launched("gg_locate_noalloc: launch of the block-sum scan failed")) return GG_ERR_CUDA;
     k_scan_add<<<(int)nblk, 1024, 0, st>>>(d_offsets, nel, sums, sums + nblk);
     if (!launched("gg_locate_noalloc: launch of the scan fix-up failed")) return GG_ERR_CUDA;
-    if (cudaMemsetAsync(counts, 0, sizeof(int32_t) * (nel + 1), st) != cudaSuccess) {
-        *msg = "gg_locate_noalloc: cudaMemsetAsync failed";
-        return GG_ERR_CUDA;
-    }
-    k_scatter<<<grid_of(n_points, 256), 256, 0, st>>>(n_points, nel, d_cell, d_offsets, counts, d_order);
+    // the points' places ride in d_cell above the element (k_locate), no second count
+    launch_scatter(n_points, nel, d_cell, d_offsets, nullptr, d_order, st);
     if (!launched("gg_locate_noalloc: launch of the scatter failed")) return GG_ERR_CUDA;
-    k_segsort_inplace<<<grid_of(nel * 32, 128), 128, 0, st>>>(nel, d_offsets, d_order, flags);
+    k_segsort<true><<<segsort_grid(nel), kSegBlock, 0, st>>>(nel, d_offsets, d_order, d_order, flags);
     if (!launched("gg_locate_noalloc: launch of the per-element sort failed")) return GG_ERR_CUDA;
     int32_t hflags[2] = {0, 0};
     if (cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
