@@ -17,14 +17,14 @@
 // touches a point again.
 //
 // Two kernels.  k_points evaluates the rheology chain per point (one thread per point, both
-// precisions of a mixed build from the same loads) and leaves c_p and the force weights in
-// point order; k_moments sums them per element, four lanes per element, each lane its own
+// precisions of a mixed build from the same loads) and leaves the viscosities in point
+// order; k_moments sums them per element, four lanes per element, each lane its own
 // accumulators over the element's points in order -- the reference's summation order, and
 // the same bits whatever the launch shape.  As one kernel (rheology into shared memory, then
 // one thread per element with all 39 accumulators) the build held 255 registers, ran 8 warps
 // per SM at 0.9 instructions per cycle and took 752 µs (FP64) + 549 µs (FP32) for 7.1 M
-// points in 64³ elements; now k_points takes 280 µs for both precisions, k_moments 166 µs
-// (FP64) and 108 µs (FP32).
+// points in 64³ elements; now k_points takes 232 µs for both precisions, k_moments 197 µs
+// (FP64) and 111 µs (FP32).
 // The element's corner terms of the K diagonal and of the force go to per-element buffers;
 // k_gather_corners sums them per node in a fixed element order, so a build gives the same
 // bits on every run.
@@ -220,23 +220,20 @@ __device__ PointOut run_rheologies(const MeshK& mk, const gg_material& m, const 
     return out;
 }
 
-// Per point: viscosity, its quadrature coefficient c_p = w_p detJ η_p (FP64, with kBoth also
-// FP32 from the FP32 rheology chain), the force weights φ_p = detJ w ρ g and
-// ψ_p = detJ w Ra T (null: zero for every point).  Bound by its loads and stores
-// (60-90 bytes per point) once enough warps cover the exponential's latency: at 255
-// registers, one block per SM, it took 651 µs for 7.1 M points; three blocks spill a little
-// in the yield laws and take 280 (two: 290), 32-bit element indices in both.
+// Per point: viscosity in FP64, with kBoth also by the FP32 rheology chain, and the
+// temperature where a force term reads it (temp null: none does).
+// Bound by its loads and stores (60-90 bytes per point) once enough warps cover the
+// exponential's latency: at 255 registers, one block per SM, it took 651 µs for 7.1 M points;
+// three blocks spill a little in the yield laws and take 232 (two took 3 % more), 32-bit element
+// indices in both.
 template <int DIM, bool kBoth>
 __global__ void __launch_bounds__(256, 3)
-k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const int32_t* __restrict__ offsets,
-         const double* __restrict__ xi_s, const int32_t* __restrict__ mat_s, const double* __restrict__ ps_s,
-         const double* __restrict__ w_s, const double* __restrict__ T, const double* __restrict__ pu,
-         const double* __restrict__ pp, int prev, double gravity, double rayleigh,
-         const gg_material* __restrict__ materials, double* __restrict__ c64, float* __restrict__ c32,
-         double* __restrict__ phi, double* __restrict__ psi, double* __restrict__ eta_s,
-         double* __restrict__ incr_s, uint8_t* __restrict__ yld_s) {
+k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const double* __restrict__ xi_s,
+         const int32_t* __restrict__ mat_s, const double* __restrict__ ps_s, const double* __restrict__ T,
+         const double* __restrict__ pu, const double* __restrict__ pp, int prev, double rayleigh,
+         const gg_material* __restrict__ materials, float* __restrict__ eta32, double* __restrict__ temp,
+         double* __restrict__ eta_s, double* __restrict__ incr_s, uint8_t* __restrict__ yld_s) {
     constexpr int NEN = 1 << DIM;
-    const double wscale = (double)(1 << DIM);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < np; i += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t pe = (uint32_t)cell_s[i], row = pe / (uint32_t)mk.n[0];
         const int ijk[3] = {(int)(pe - row * (uint32_t)mk.n[0]), (int)(row % (uint32_t)mk.n[1]),
@@ -247,9 +244,6 @@ k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const int32_t
         const gg_material& m = materials[mat_s[i]];
         const double ps = ps_s[i];
         const PointOut po = run_rheologies<DIM, double>(mk, m, ijk, pe, xi, T, pu, pp, ps, prev);
-        // per-point weight (DVCWeights) or _ConstantWeights_Calculate
-        const double w = w_s ? w_s[i] : wscale / (double)(offsets[pe + 1] - offsets[pe]);
-        c64[i] = (w * mk.detJ) * po.eta;
         eta_s[i] = po.eta;
         incr_s[i] = po.incr;
         yld_s[i] = po.yielded;
@@ -257,43 +251,43 @@ k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const int32_t
             float x32[3] = {0.f, 0.f, 0.f};
 #pragma unroll
             for (int d = 0; d < DIM; d++) x32[d] = (float)xi[d];
-            const PointOut pf = run_rheologies<DIM, float>(mk, m, ijk, pe, x32, T, pu, pp, ps, prev);
-            c32[i] = (float)(w * mk.detJ) * (float)pf.eta;
+            eta32[i] = (float)run_rheologies<DIM, float>(mk, m, ijk, pe, x32, T, pu, pp, ps, prev).eta;
         }
-        if (phi || psi) {
+        if (temp) {
             double Tp = 0.0;
-            if (T && (rayleigh != 0.0 || m.alpha != 0.0)) {
+            if (rayleigh != 0.0 || m.alpha != 0.0) {
                 double N[NEN];
                 shape<DIM, double>(xi, N);
 #pragma unroll
                 for (int a = 0; a < NEN; a++) Tp += T[elem_node<DIM>(mk, ijk, a)] * N[a];
             }
-            if (phi) {
-                const double rho = m.density * (1.0 - m.alpha * Tp);
-                phi[i] = mk.detJ * w * rho * gravity;
-            }
-            if (psi) psi[i] = mk.detJ * w * (rayleigh * Tp);
+            temp[i] = Tp;
         }
     }
 }
 
-// Per element, four lanes: lane q < 3 sums the moments of ξ-exponent q (every lane the same
-// instructions, with its own power of ξ), lane q the force terms of corners q·NC … (φ, ψ
-// null: none).  Then every lane takes all moments and forms its corners' diagonal terms.
+// Per element, four lanes, over its points in order: c_p = w_p detJ η_p and the force weights
+// φ_p = detJ w ρ g, ψ_p = detJ w Ra T are formed on the way; lane q < 3 sums the moments of
+// ξ-exponent q (every lane the same instructions, with its own power of ξ), lane q the force
+// terms of corners q·NC ….  want_phi 0 / temp null: those weights are zero for every point.
+// Then every lane takes all moments and forms its corners' diagonal terms.
 // Eight elements per warp keep an SM at 32 and more warps, where one thread per element and
 // 39 accumulators left 8; the eight streams of points of a warp meet in L1.
 template <int DIM, typename R, bool kForce>
 __global__ void __launch_bounds__(128)
 k_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets, const double* __restrict__ xi_s, int64_t np,
-          const R* __restrict__ cp, const double* __restrict__ phi, const double* __restrict__ psi,
-          R* __restrict__ mom, R* __restrict__ kcorner, double* __restrict__ sdiag, double* __restrict__ fcorner,
-          int32_t* __restrict__ flag) {
+          const R* __restrict__ eta, const double* __restrict__ w_s, const int32_t* __restrict__ mat_s,
+          const double* __restrict__ temp, const gg_material* __restrict__ materials, int want_phi, double gravity,
+          double rayleigh, R* __restrict__ mom, R* __restrict__ kcorner, double* __restrict__ sdiag,
+          double* __restrict__ fcorner, int32_t* __restrict__ flag) {
     constexpr unsigned kFull = 0xffffffffu;
     constexpr int NM = n_moments<DIM>(), NEN = 1 << DIM, NC = NEN / 4, NZ = DIM == 3 ? 3 : 1;
     const int q = threadIdx.x & 3;
     const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     const bool own = e < nel;
     const int32_t b = own ? offsets[e] : 0, en = own ? offsets[e + 1] : 0;
+    // _ConstantWeights_Calculate, or the per-point weight (DVCWeights)
+    const double wconst = (double)(1 << DIM) / (double)(en - b);
     R acc[3][NZ];
 #pragma unroll
     for (int bb = 0; bb < 3; bb++)
@@ -305,7 +299,8 @@ k_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets, const doub
 #pragma unroll 4
     for (int32_t i = b; i < en; i++) {
         const double xd = xi_s[i], yd = xi_s[np + i], zd = DIM == 3 ? xi_s[2 * np + i] : 0.0;
-        const R c = cp[i], x = (R)xd, y = (R)yd, z = (R)zd;
+        const double w = w_s ? w_s[i] : wconst;
+        const R c = (R)(w * mk.detJ) * eta[i], x = (R)xd, y = (R)yd, z = (R)zd;
         const R px = q == 0 ? R(1) : q == 1 ? x : x * x;
         const R pxy[3] = {px, px * y, px * (y * y)};
         const R zz = z * z;
@@ -318,7 +313,14 @@ k_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets, const doub
             }
         }
         if (kForce) {
-            const double ph = phi ? phi[i] : 0.0, ps = psi ? psi[i] : 0.0;
+            const double Tp = temp ? temp[i] : 0.0;
+            double ph = 0.0;
+            if (want_phi) {
+                const gg_material& m = materials[mat_s[i]];
+                const double rho = m.density * (1.0 - m.alpha * Tp);
+                ph = mk.detJ * w * rho * gravity;
+            }
+            const double ps = temp ? mk.detJ * w * (rayleigh * Tp) : 0.0;
 #pragma unroll
             for (int j = 0; j < NC; j++) {
                 const int a = q * NC + j;
@@ -499,29 +501,30 @@ static void launch_build(Handle& H, bool mixed, int prev, const double* pu, cons
     cudaStream_t st = H.stream;
     const double* T = H.has_T ? H.T.as<double>() : nullptr;
     const double* w = H.weights.mode == GG_WEIGHTS_DVC && H.dvc_valid ? H.w_s.as<double>() : nullptr;
-    double* phi = phi_nonzero(H) ? H.pt_phi.as<double>() : nullptr;
-    double* psi = psi_nonzero(H) ? H.pt_psi.as<double>() : nullptr;
-    double* c64 = H.pt_c64.as<double>();
-    float* c32 = mixed ? H.pt_c32.as<float>() : nullptr;
+    double* temp = psi_nonzero(H) ? H.pt_temp.as<double>() : nullptr;
+    // the points' elements in input order are not read again after gg_locate: their words
+    // hold the FP32 viscosities
+    float* eta32 = mixed ? H.cell.as<float>() : nullptr;
     auto points = [&](auto kernel) {
-        kernel<<<grid_for(np, 256), 256, 0, st>>>(
-            H.mk, np, H.cell_s.as<int32_t>(), H.offsets.as<int32_t>(), H.xi_s.as<double>(), H.mat_s.as<int32_t>(),
-            H.ps_s.as<double>(), w, T, pu, pp, prev, H.force.gravity, H.force.rayleigh, H.d_materials.as<gg_material>(),
-            c64, c32, phi, psi, H.eta_s.as<double>(), H.incr_s.as<double>(), H.yld_s.as<uint8_t>());
+        kernel<<<grid_for(np, 256), 256, 0, st>>>(H.mk, np, H.cell_s.as<int32_t>(), H.xi_s.as<double>(),
+                                                  H.mat_s.as<int32_t>(), H.ps_s.as<double>(), T, pu, pp, prev,
+                                                  H.force.rayleigh, H.d_materials.as<gg_material>(), eta32, temp,
+                                                  H.eta_s.as<double>(), H.incr_s.as<double>(), H.yld_s.as<uint8_t>());
         GG_CUDA(cudaGetLastError());
     };
     if (mixed) points(k_points<DIM, true>);
     else points(k_points<DIM, false>);
     const unsigned grid = (unsigned)((4 * nel + 127) / 128);
     k_moments<DIM, double, true><<<grid, 128, 0, st>>>(
-        H.mk, nel, H.offsets.as<int32_t>(), H.xi_s.as<double>(), np, c64, phi, psi, H.mom64.as<double>(),
+        H.mk, nel, H.offsets.as<int32_t>(), H.xi_s.as<double>(), np, H.eta_s.as<double>(), w, H.mat_s.as<int32_t>(),
+        temp, H.d_materials.as<gg_material>(), phi_nonzero(H), H.force.gravity, H.force.rayleigh, H.mom64.as<double>(),
         H.kcorner.as<double>(), H.sdiag.as<double>(), H.fcorner.as<double>(), H.flag.as<int32_t>());
     GG_CUDA(cudaGetLastError());
     gather_corners<DIM, double>(H, H.kdiag64.as<double>(), H.f.as<double>());
     if (mixed) {
         k_moments<DIM, float, false><<<grid, 128, 0, st>>>(
-            H.mk, nel, H.offsets.as<int32_t>(), H.xi_s.as<double>(), np, c32, nullptr, nullptr, H.mom32.as<float>(),
-            H.kcorner.as<float>(), nullptr, nullptr, H.flag.as<int32_t>());
+            H.mk, nel, H.offsets.as<int32_t>(), H.xi_s.as<double>(), np, eta32, w, nullptr, nullptr, nullptr, 0, 0.0, 0.0,
+            H.mom32.as<float>(), H.kcorner.as<float>(), nullptr, nullptr, H.flag.as<int32_t>());
         GG_CUDA(cudaGetLastError());
         gather_corners<DIM, float>(H, H.kdiag32.as<float>(), nullptr);
     }
@@ -544,11 +547,8 @@ int build_operator(Handle& H, int precision, int prev, const double* d_prev_u,
     upload_materials(H);
     GG_CUDA(cudaMemsetAsync(H.flag.p, 0, sizeof(int32_t) * 4, st));
     const bool mixed = precision == GG_PRECISION_MIXED;
-    H.pt_c64.ensure(sizeof(double) * H.np_in);
-    if (phi_nonzero(H)) H.pt_phi.ensure(sizeof(double) * H.np_in);
-    if (psi_nonzero(H)) H.pt_psi.ensure(sizeof(double) * H.np_in);
+    if (psi_nonzero(H)) H.pt_temp.ensure(sizeof(double) * H.np_in);
     if (mixed) {
-        H.pt_c32.ensure(sizeof(float) * H.np_in);
         H.mom32.ensure(sizeof(float) * nm * nel);
         H.kdiag32.ensure(sizeof(float) * nd);
     }

@@ -101,7 +101,7 @@ struct Handle {
 
     // operator
     DBuf mom64, mom32, kdiag64, kdiag32, sdiag, hvec, f;
-    DBuf pt_c64, pt_c32, pt_phi, pt_psi;  // per-point quadrature and force weights (build scratch)
+    DBuf pt_temp;           // temperature at the points (build scratch)
     DBuf kcorner, fcorner;  // per-element corner terms of the diagonal / force (build scratch)
     bool built = false;
     int built_precision = -1;
