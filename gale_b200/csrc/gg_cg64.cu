@@ -10,14 +10,14 @@
 //             and the element energies pᵀK_e p;
 //   nodes     α, each node adds its 2^dim element terms in class order (the sum the class
 //             launches form), x, r, z, p, and the two dot products;
-// so an iteration is two barriers.  Small meshes run in one thread-block cluster, whose
-// hardware barrier orders the 16 CTAs' global writes in a fraction of a grid barrier;
-// larger ones run as a cooperative grid with the counter barrier of gg_grid.cuh.
+// so an iteration is two barriers.  2D meshes of up to about 64² run in the shared memory of
+// one thread-block cluster (k_cg64_strip); others as a cooperative grid with the counter
+// barrier of gg_grid.cuh (k_cg64).
 // Every sum keeps the order of the launches it replaces (gg_solve.cu: 592 blocks of 256
 // threads over the vectors, one block per 256-element tile of a class): the partial sums are
 // formed per such block, by whichever CTA has it, and added in block index order by every
 // CTA, so a solve gives the same bits on every run, for any number of CTAs.  Per iteration:
-// 5.2 µs on 32², 7.2 on 64² and 128², 13 on 16³, 19 on 32³, 38 on 48³ (60 as launches).
+// 5.0 µs on 32², 5.1 on 64², 7.2 on 128², 13 on 16³, 19 on 32³, 38 on 48³ (60 as launches).
 #include <math.h>
 
 #include <algorithm>
@@ -34,6 +34,7 @@ namespace {
 
 constexpr int kVecBlocks = 592;  // blocks of 256 threads the vector sums are split over
 constexpr int kCluster = 16;
+constexpr int kStripSmem = 222 * 1024;
 constexpr int64_t kTermBytes = int64_t(32) << 20;  // element terms that stay in L2
 
 struct Cg64Args {
@@ -84,18 +85,6 @@ __device__ __forceinline__ void group_sum(double (&v)[NV], int g) {
     group_bar(g);
 #pragma unroll
     for (int k = 0; k < NV; k++) v[k] = s_tot[g][k];
-}
-
-template <bool kUseCluster>
-__device__ __forceinline__ bool all_sync(GridBarrier* gb, unsigned int* epoch) {
-    if constexpr (kUseCluster) {
-        (void)gb;
-        (void)epoch;
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        return true;
-    } else {
-        return grid_barrier(gb, epoch);
-    }
 }
 
 // element of thread t in tile `tile` of class `color` (apply_tiles_class)
@@ -156,7 +145,7 @@ __device__ __forceinline__ NodeAt<DIM> node_at(const Cg64Args& A, int64_t at) {
     return q;
 }
 
-template <int DIM, bool kUseCluster>
+template <int DIM>
 __global__ void __launch_bounds__(cg64_threads<DIM>(), 1) k_cg64(const __grid_constant__ Cg64Args A) {
     constexpr int NS = 1 << DIM, NM = n_moments<DIM>();
     const MeshK& mk = A.mk;
@@ -195,7 +184,7 @@ __global__ void __launch_bounds__(cg64_threads<DIM>(), 1) k_cg64(const __grid_co
             A.part_n[A.vec_blocks + vb] = acc[1];
         }
     }
-    if (!all_sync<kUseCluster>(A.gb, &epoch)) return;
+    if (!grid_barrier(A.gb, &epoch)) return;
     auto vec_sums = [&](double (&v)[2]) {
         v[0] = v[1] = 0.0;
         for (int b = t; b < A.vec_blocks; b += 256) {
@@ -274,7 +263,7 @@ __global__ void __launch_bounds__(cg64_threads<DIM>(), 1) k_cg64(const __grid_co
                 break;
             }
         }
-        if (!all_sync<kUseCluster>(A.gb, &epoch)) return;
+        if (!grid_barrier(A.gb, &epoch)) return;
         // ---- nodes.  The loads of the first entry do not depend on α
         double ye[NS], rv = 0.0, zv = 0.0, pv = 0.0, xv = 0.0;
         auto load_node = [&](const NodeAt<DIM>& q, int64_t i) {
@@ -324,7 +313,7 @@ __global__ void __launch_bounds__(cg64_threads<DIM>(), 1) k_cg64(const __grid_co
                 A.part_n[A.vec_blocks + vb] = acc[1];
             }
         }
-        if (!all_sync<kUseCluster>(A.gb, &epoch)) return;
+        if (!grid_barrier(A.gb, &epoch)) return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.s->rnorm0 = rnorm0;
@@ -336,55 +325,489 @@ __global__ void __launch_bounds__(cg64_threads<DIM>(), 1) k_cg64(const __grid_co
     }
 }
 
-int cluster_fits(const void* fn, int threads) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kCluster);
-    cfg.blockDim = dim3(threads);
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kCluster;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
+// ---- 2D meshes whose strips fit the shared memory of one cluster ------------------------
+// The same two phases with everything in shared memory: CTA s of the cluster owns the element
+// rows R_s … R_{s+1} − 1 (even R_s, so every parity class keeps whole rows) and, of the vector
+// entries, an equal share of the 32-entry chunks at about the same nodes.  A phase writes what the next
+// one reads straight into the reader's shared memory: an element its corner terms to the CTA
+// that sums that entry, an entry its z and p to the one or two strips whose elements use its
+// node -- nearly always the CTA itself, where a plain store does (a store through the cluster
+// window moves some 16 bytes per cycle and CTA, and 18 warps that each stored their sums to
+// 16 CTAs took 2000 cycles).  The partial sums go to every CTA in one contiguous piece per
+// destination.  An iteration is then two cluster barriers of 450 cycles, the two divisions,
+// the sums, and no load from L2: 5.0 µs on 20² to 48², 5.1 on 64², where the grid form takes
+// 7.0-7.6 and the captured launches 22-24.  What is left is the instruction latency of the
+// one warp per scheduler that has work (the element term alone is 1400 cycles).
+// The sums: a warp of k_cg64's 256-thread blocks is one class row segment of 32 elements, or
+// one chunk of 32 vector entries, so the partial sums exchanged are those of the warps, and
+// they are added up in block_sum's order.
+constexpr int kStripThreads = 576;  // 18 warps of ≤ 112 registers: a 64² strip has 17-18 chunks
+constexpr unsigned kNoAddr = 0xffffffffu;
+constexpr unsigned kRemote = 0x80000000u;  // marks an address in another CTA (cluster addresses stay below)
+
+struct Cg64Strip {
+    int cluster;
+    int row[kCluster + 1];              // first element row of every strip
+    int max_tasks, max_chunks, max_nl;  // array extents, the same in every CTA
+    int units, vec_blocks;              // element tiles, vector blocks of 256
+    // byte offsets in shared memory
+    int zl, pl, terms, x, r, d, z, p, mom, taddr, zaddr, ex, nx, ei, ni, bytes;
+};
+
+__device__ __forceinline__ unsigned shared_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+// address of p in the cluster's CTA `rank`; in this CTA (`me`) the plain shared address, which
+// lies below the cluster window's per-CTA stride
+__device__ __forceinline__ unsigned cluster_addr(const void* p, int rank, int me) {
+    const unsigned a = shared_addr(p);
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return rank == me ? a : (r | kRemote);
+}
+__device__ __forceinline__ void cluster_store(unsigned a, double v) {
+    asm volatile(
+        "{\n\t.reg .pred r;\n\t.reg .b32 t;\n\t"
+        "setp.lt.s32 r, %0, 0;\n\tand.b32 t, %0, 0x7fffffff;\n\t"
+        "@r st.shared::cluster.f64 [t], %1;\n\t@!r st.shared::cta.f64 [t], %1;\n\t}" ::"r"(a),
+        "d"(v)
+        : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// CTA s owns the chunks of component c that begin at nodes s·nnode/cluster … (equal shares, so
+// the last strip's extra node row makes no CTA wait); the first of them
+__device__ __forceinline__ int chunk_lo(const MeshK& mk, const Cg64Strip& S, int s, int c) {
+    return (int)((c * mk.nnode + s * mk.nnode / S.cluster + 31) >> 5);
+}
+__device__ __forceinline__ int chunk_owner(const MeshK& mk, const Cg64Strip& S, int node) {
+    int s = 0;
+    while (s + 1 < S.cluster && node >= (int)((s + 1) * mk.nnode / S.cluster)) s++;
+    return s;
+}
+// strip of a node row
+__device__ __forceinline__ int strip_of(const Cg64Strip& S, int node_row) {
+    int s = 0;
+    while (s + 1 < S.cluster && node_row >= S.row[s + 1]) s++;
+    return s;
+}
+
+// Sum over up to 256 blocks of NV values, each block the block_sum of its 8 warps' partial
+// sums v[idx[8b + w]], as the last block of a 256-thread launch forms it: a CTA warp per launch warp, then
+// every thread adds up the warps.  stage: [8·NV] doubles, zero past the launch's warps; the
+// CTA meets once.
+template <int NV>
+__device__ __forceinline__ void cta_total(const double* v, const uint16_t* idx, int blocks, double* stage,
+                                          double (&tot)[NV]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (32 * warp < blocks) {
+        const uint4 at = *reinterpret_cast<const uint4*>(idx + 8 * threadIdx.x);  // a zero past the blocks
+        const uint32_t pair[4] = {at.x, at.y, at.z, at.w};
+        double p[8][NV], s[NV];
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            const int q = (pair[w >> 1] >> (16 * (w & 1))) & 0xffff;
+#pragma unroll
+            for (int k = 0; k < NV; k++) p[w][k] = v[q * NV + k];
+        }
+#pragma unroll
+        for (int k = 0; k < NV; k++)
+            s[k] = ((p[0][k] + p[4][k]) + (p[2][k] + p[6][k])) + ((p[1][k] + p[5][k]) + (p[3][k] + p[7][k]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < NV; k++) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < NV; k++) stage[8 * k + warp] = s[k];
     }
-    return n;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        const double* t = stage + 8 * k;
+        tot[k] = ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
+    }
+}
+
+__global__ void __launch_bounds__(kStripThreads, 1)
+k_cg64_strip(const __grid_constant__ Cg64Args A, const __grid_constant__ Cg64Strip S) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ double stage_n[16], stage_e[8];
+    __shared__ int s_stop;  // 0 go on, 1 converged, 2 iteration limit, 3 not finite
+    constexpr int NS = 4, NM = 6, kWarps = kStripThreads / 32;
+    static_assert(kWarps >= kCluster, "a warp per destination");
+    const MeshK& mk = A.mk;
+    const int nnode = (int)mk.nnode, n = 2 * nnode, nn0 = mk.nn[0];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int me = blockIdx.x;  // one cluster: the CTA's rank in it
+    const int r0 = S.row[me], r1 = S.row[me + 1];
+    // [2][max_nl]: node rows r0 … r1, the even nodes of a row before the odd ones, so that the
+    // elements of a class read neighbouring words
+    double* zl = reinterpret_cast<double*>(sm + S.zl);
+    const int half = (nn0 + 1) / 2;
+    double* pl = reinterpret_cast<double*>(sm + S.pl);
+    double* terms = reinterpret_cast<double*>(sm + S.terms);  // [4 classes][32·max_chunks]
+    double* xs = reinterpret_cast<double*>(sm + S.x);         // the CTA's entries
+    double* rs = reinterpret_cast<double*>(sm + S.r);
+    double* ds = reinterpret_cast<double*>(sm + S.d);
+    double* zs = reinterpret_cast<double*>(sm + S.z);
+    double* ps = reinterpret_cast<double*>(sm + S.p);
+    double* mom = reinterpret_cast<double*>(sm + S.mom);          // [6][32·max_tasks]
+    unsigned* taddr = reinterpret_cast<unsigned*>(sm + S.taddr);  // [8][32·max_tasks]
+    unsigned* zaddr = reinterpret_cast<unsigned*>(sm + S.zaddr);  // [2][32·max_chunks], then: entry fixed or missing
+    // partial sums of every CTA: element tasks [cluster][max_tasks], chunks
+    // [cluster][max_chunks][2], a zero behind each; where those of a block's 8 warps are
+    double* ex = reinterpret_cast<double*>(sm + S.ex);
+    double* nx = reinterpret_cast<double*>(sm + S.nx);
+    uint16_t* ei = reinterpret_cast<uint16_t*>(sm + S.ei);  // [units][8]
+    uint16_t* ni = reinterpret_cast<uint16_t*>(sm + S.ni);  // [vec_blocks][8]
+    const int te_n = 32 * S.max_tasks, ts_n = 32 * S.max_chunks;
+    // this CTA's chunks: component 0, then component 1
+    const int q0 = chunk_lo(mk, S, me, 0), c0n = chunk_lo(mk, S, me + 1, 0) - q0;
+    const int q1 = chunk_lo(mk, S, me, 1), chunks = c0n + chunk_lo(mk, S, me + 1, 1) - q1;
+    // its element tasks: (class row pair of the strip, class, segment of 32)
+    const int ntx0 = ((mk.n[0] + 1) / 2 + 31) / 32, tasks = (r1 - r0 + 1) / 2 * 4 * ntx0;
+    const unsigned off_pl = (unsigned)(S.pl - S.zl);
+
+    // ---- tables
+    for (int i = threadIdx.x; i < 4 * ts_n; i += kStripThreads) terms[i] = 0.0;
+    for (int i = threadIdx.x; i < 8 * ((S.units + 31) & ~31); i += kStripThreads) ei[i] = (uint16_t)(S.cluster * S.max_tasks);
+    for (int i = threadIdx.x; i < 8 * ((S.vec_blocks + 31) & ~31); i += kStripThreads) ni[i] = (uint16_t)(S.cluster * S.max_chunks);
+    if (threadIdx.x < 16) stage_n[threadIdx.x] = 0.0;
+    if (threadIdx.x < 8) stage_e[threadIdx.x] = 0.0;
+    if (threadIdx.x == 0) {
+        ex[S.cluster * S.max_tasks] = 0.0;
+        nx[2 * S.cluster * S.max_chunks] = nx[2 * S.cluster * S.max_chunks + 1] = 0.0;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < S.cluster * S.max_tasks; i += kStripThreads) {
+        // tile of the class row: rows in eights, segments of the class's own width
+        const int s = i / S.max_tasks, task = i - s * S.max_tasks;
+        const int seg = task % ntx0, color = (task / ntx0) & 3, cj = S.row[s] / 2 + task / (4 * ntx0);
+        const int ntx = (class_extent<2>(mk, 0, color) + 31) / 32;
+        if (task < (S.row[s + 1] - S.row[s] + 1) / 2 * 4 * ntx0 && seg < ntx)
+            ei[8 * (color * A.tiles + (cj >> 3) * ntx + seg) + (cj & 7)] = (uint16_t)i;
+    }
+    for (int i = threadIdx.x; i < S.cluster * S.max_chunks; i += kStripThreads) {
+        const int s = i / S.max_chunks, slot = i - s * S.max_chunks;
+        const int a0 = chunk_lo(mk, S, s, 0), n0 = chunk_lo(mk, S, s + 1, 0) - a0;
+        const int a1 = chunk_lo(mk, S, s, 1), n1 = chunk_lo(mk, S, s + 1, 1) - a1;
+        if (slot < n0 + n1) ni[slot < n0 ? a0 + slot : a1 + slot - n0] = (uint16_t)i;
+    }
+    for (int te = threadIdx.x; te < te_n; te += kStripThreads) {
+        const int task = te >> 5, seg = task % ntx0, color = (task / ntx0) & 3, cj = r0 / 2 + task / (4 * ntx0);
+        const int i = 2 * (32 * seg + (te & 31)) + (color & 1), j = 2 * cj + (color >> 1);
+        const bool on = task < tasks && i < mk.n[0] && j < r1;
+        for (int a = 0; a < NS; a++) {
+            const int node = i + (a & 1) + nn0 * (j + (a >> 1));
+            for (int c = 0; c < 2; c++) {
+                unsigned t = kNoAddr;
+                if (on) {
+                    const int at = c * nnode + node, q = at >> 5, first = q << 5;
+                    const int fc = first >= nnode ? 1 : 0, s = chunk_owner(mk, S, first - fc * nnode);
+                    const int lo = chunk_lo(mk, S, s, 0);
+                    const int slot = fc == 0 ? q - lo : chunk_lo(mk, S, s + 1, 0) - lo + q - chunk_lo(mk, S, s, 1);
+                    t = cluster_addr(terms + color * ts_n + slot * 32 + (at & 31), s, me);
+                }
+                taddr[(a * 2 + c) * te_n + te] = t;
+            }
+        }
+        if (on)
+            for (int k = 0; k < NM; k++) mom[k * te_n + te] = A.mom[(int64_t)k * mk.nel + i + mk.n[0] * j];
+    }
+    for (int ts = threadIdx.x; ts < ts_n; ts += kStripThreads) {
+        const int slot = ts >> 5, at = 32 * (slot < c0n ? q0 + slot : q1 + slot - c0n) + (ts & 31);
+        unsigned t0 = kNoAddr, t1 = kNoAddr;
+        if (slot < chunks && at < n) {
+            const int c = at >= nnode, node = at - c * nnode, row = node / nn0, s = strip_of(S, row);
+            const int col = node % nn0, at_l = c * S.max_nl + (col & 1) * half + (col >> 1);
+            t0 = cluster_addr(zl + at_l + (row - S.row[s]) * nn0, s, me);
+            if (s > 0 && row == S.row[s])
+                t1 = cluster_addr(zl + at_l + (row - S.row[s - 1]) * nn0, s - 1, me);
+        }
+        zaddr[ts] = t0;
+        zaddr[ts_n + ts] = t1;
+    }
+    cluster_barrier();  // every CTA's arrays exist and are zeroed
+    // z and p of entry ts to the strips that gather it
+    auto publish = [&](int ts, double zv, double pv) {
+        const unsigned t0 = zaddr[ts], t1 = zaddr[ts_n + ts];
+        if (t0 != kNoAddr) {
+            cluster_store(t0, zv);
+            cluster_store(t0 + off_pl, pv);
+        }
+        if (t1 != kNoAddr) {
+            cluster_store(t1, zv);
+            cluster_store(t1 + off_pl, pv);
+        }
+    };
+    // this CTA's `count` doubles at own[0 …] to the same place of every other CTA, a warp each
+    auto share = [&](const double* own, int count) {
+        __syncthreads();
+        if (warp < S.cluster && warp != me) {
+            const unsigned t = cluster_addr(own, warp, me);
+            for (int k = lane; k < count; k += 32) cluster_store(t + 8u * (unsigned)k, own[k]);
+        }
+    };
+    double* own_n = nx + 2 * me * S.max_chunks;
+    double* own_e = ex + me * S.max_tasks;
+    // the two sums of the warp's chunk
+    auto chunk_sums = [&](int slot, double a, double b) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+        }
+        if (lane == 0) {
+            own_n[2 * slot] = a;
+            own_n[2 * slot + 1] = b;
+        }
+    };
+    for (int slot = warp; slot < chunks; slot += kWarps) {
+        const int ts = slot * 32 + lane, at = 32 * (slot < c0n ? q0 + slot : q1 + slot - c0n) + lane;
+        double zz = 0.0, rz = 0.0, rv = 0.0, zv = 0.0, dv = 1.0;
+        bool fixed = true;
+        if (at < n) {
+            const int c = at >= nnode;
+            fixed = (A.bc[at - c * nnode] >> c) & 1;
+            if (!fixed) {
+                dv = A.diag[at];
+                rv = A.b[at];
+                zv = rv / dv;
+            }
+            zz = zv * zv;
+            rz = rv * zv;
+        }
+        xs[ts] = 0.0;
+        rs[ts] = rv;
+        ds[ts] = dv;
+        zs[ts] = zv;
+        ps[ts] = 0.0;
+        zaddr[2 * ts_n + ts] = fixed;
+        publish(ts, zv, 0.0);
+        chunk_sums(slot, zz, rz);
+    }
+    share(own_n, 2 * chunks);
+    cluster_barrier();
+
+    // local node of a task's element, and what does not change over the iterations
+    auto elem_nz = [&](int task) {
+        const int seg = task % ntx0, color = (task / ntx0) & 3, lp = task / (4 * ntx0);
+        const int px = color & 1;  // its corner 0; the next node of the row: (see load_elem)
+        return 32 * seg + lane + px * half + nn0 * (2 * lp + (color >> 1));
+    };
+    const int first_nz = elem_nz(warp);
+    const bool first_on = warp < tasks && taddr[warp * 32 + lane] != kNoAddr;
+
+    double beta = 0.0, rz = 0.0, rnorm = 0.0, rnorm0 = 0.0, ttol = 0.0, pAp = 0.0;
+    int it = 0, failed = 0;
+    bool started = false;
+    for (;;) {
+        // ---- elements (the first task's loads do not wait for β)
+        double zz[2][NS], pp[2][NS], M[NM];
+        auto load_elem = [&](int nz, int task, int te) {
+            // the odd neighbour of an even node, the even neighbour of an odd one
+            const int dx = ((task / ntx0) & 1) ? 1 - half : half;
+#pragma unroll
+            for (int c = 0; c < 2; c++)
+#pragma unroll
+                for (int a = 0; a < NS; a++) {
+                    const int at = c * S.max_nl + nz + (a & 1) * dx + nn0 * (a >> 1);
+                    zz[c][a] = zl[at];
+                    pp[c][a] = pl[at];
+                }
+#pragma unroll
+            for (int k = 0; k < NM; k++) M[k] = mom[k * te_n + te];
+        };
+        if (first_on) load_elem(first_nz, warp, warp * 32 + lane);
+        double sums[2];
+        cta_total<2>(nx, ni, S.vec_blocks, stage_n, sums);
+        if (started) beta = sums[1] / rz;
+        rz = sums[1];
+        for (int task = warp; task < tasks; task += kWarps) {
+            const int te = task * 32 + lane;
+            const bool on = task == warp ? first_on : taddr[te] != kNoAddr;
+            if (on && task != warp) load_elem(elem_nz(task), task, te);
+            double en = 0.0;
+            if (on) {
+                double m[2][NS];
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+#pragma unroll
+                    for (int a = 0; a < NS; a++) m[c][a] = zz[c][a] + beta * pp[c][a];
+                en = element_compute<2, double, true>(mk, m, M, -1, [&](int c, int a, double v) {
+                    cluster_store(taddr[(a * 2 + c) * te_n + te], v);
+                });
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) en += __shfl_xor_sync(0xffffffffu, en, o);
+            if (lane == 0) own_e[task] = en;
+        }
+        if (warp == kWarps - 1) {
+            // the stopping test, by the warp that has the fewest tasks
+            rnorm = sqrt(sums[0]);
+            if (!started) {
+                rnorm0 = rnorm;
+                const double tt = A.rtol * rnorm0;
+                ttol = tt < 1e-50 ? 1e-50 : tt;
+            }
+            const int done = it + (started ? 1 : 0);
+            if (lane == 0)
+                s_stop = started && (!(rnorm == rnorm) || isinf(rnorm)) ? 3
+                         : rnorm <= ttol                                ? 1
+                         : started && done >= A.maxit                   ? 2
+                                                                        : 0;
+        }
+        share(own_e, tasks);
+        if (started) it++;
+        started = true;
+        if (s_stop) {
+            failed = s_stop - 1;
+            break;
+        }
+        cluster_barrier();
+        // ---- nodes (the first chunk's loads do not wait for α)
+        double ye[NS], rv, xv, zv, pv;
+        auto load_node = [&](int ts) {
+#pragma unroll
+            for (int k = 0; k < NS; k++) ye[k] = terms[k * ts_n + ts];
+            rv = rs[ts];
+            xv = xs[ts];
+            zv = zs[ts];
+            pv = ps[ts];
+        };
+        if (warp < chunks) load_node(warp * 32 + lane);
+        double e[1];
+        cta_total<1>(ex, ei, S.units, stage_e, e);
+        pAp = e[0];
+        const double alpha = rz / pAp;
+        if (!(pAp > 0.0) || isinf(pAp)) {
+            failed = 3;
+            break;
+        }
+        for (int slot = warp; slot < chunks; slot += kWarps) {
+            const int ts = slot * 32 + lane;
+            if (slot != warp) load_node(ts);
+            const bool fixed = zaddr[2 * ts_n + ts] != 0u;
+            double ap = 0.0;
+#pragma unroll
+            for (int k = 0; k < NS; k++) ap += ye[k];
+            const double pnew = zv + beta * pv;
+            xs[ts] = xv + alpha * pnew;
+            const double rn = fixed ? 0.0 : rv - alpha * ap;
+            const double zn = fixed ? 0.0 : rn / ds[ts];
+            rs[ts] = rn;
+            zs[ts] = zn;
+            ps[ts] = pnew;
+            publish(ts, zn, pnew);
+            chunk_sums(slot, zn * zn, rn * zn);
+        }
+        share(own_n, 2 * chunks);
+        cluster_barrier();
+    }
+    cluster_barrier();  // no CTA leaves while another may still write into it
+    for (int slot = warp; slot < chunks; slot += kWarps) {
+        const int at = 32 * (slot < c0n ? q0 + slot : q1 + slot - c0n) + lane;
+        if (at < n) A.x[at] = xs[slot * 32 + lane];
+    }
+    if (me == 0 && threadIdx.x == kStripThreads - 32) {
+        A.s->rnorm0 = rnorm0;
+        A.s->rnorm = rnorm;
+        A.s->pAp = pAp;
+        A.s->iterations = it;
+        A.s->failed = failed;
+        A.s->done = 1;
+    }
+}
+
+// Launch of the strip kernel; false where the mesh or the device does not allow it.
+bool run_strip(Handle& H, const Cg64Args& A) {
+    const MeshK& mk = H.mk;
+    Cg64Strip S;
+    std::memset(&S, 0, sizeof S);
+    const int ny = mk.n[1], nn0 = mk.nn[0], pairs = (ny + 1) / 2;
+    S.cluster = 1;
+    while (2 * S.cluster <= kCluster && 2 * S.cluster <= pairs) S.cluster *= 2;
+    for (int s = 0; s < S.cluster; s++) S.row[s] = 2 * (int)((int64_t)s * pairs / S.cluster);
+    S.row[S.cluster] = ny;
+    const int64_t nnode = mk.nnode;
+    auto lo = [&](int s, int c) {
+        return (c * nnode + s * nnode / S.cluster + 31) / 32;
+    };
+    int64_t tasks = 0, chunks = 0, nl = 0;
+    for (int s = 0; s < S.cluster; s++) {
+        const int rows = S.row[s + 1] - S.row[s];
+        tasks = std::max<int64_t>(tasks, (int64_t)((rows + 1) / 2) * 4 * (((mk.n[0] + 1) / 2 + 31) / 32));
+        chunks = std::max(chunks, lo(s + 1, 0) - lo(s, 0) + lo(s + 1, 1) - lo(s, 1));
+        nl = std::max<int64_t>(nl, (int64_t)(rows + 1) * nn0);
+    }
+    int64_t at = 0;
+    auto take = [&](int64_t bytes) {
+        const int64_t r = at;
+        at += (bytes + 15) / 16 * 16;
+        return (int)std::min<int64_t>(r, 1 << 30);
+    };
+    const int64_t d = sizeof(double), te = 32 * tasks, ts = 32 * chunks;
+    S.units = 4 * A.tiles;
+    S.vec_blocks = A.vec_blocks;
+    S.zl = take(2 * nl * d);
+    S.pl = take(2 * nl * d);
+    S.terms = take(4 * ts * d);
+    S.x = take(ts * d);
+    S.r = take(ts * d);
+    S.d = take(ts * d);
+    S.z = take(ts * d);
+    S.p = take(ts * d);
+    S.mom = take(6 * te * d);
+    S.taddr = take(8 * te * 4);
+    S.zaddr = take(3 * ts * 4);
+    S.ex = take((S.cluster * tasks + 1) * d);
+    S.nx = take((S.cluster * chunks + 1) * 2 * d);
+    S.ei = take(8 * (int64_t)((S.units + 31) & ~31) * 2);  // whole warps read them
+    S.ni = take(8 * (int64_t)((S.vec_blocks + 31) & ~31) * 2);
+    // a second round of chunks costs what the cluster gains: 72² (21 chunks per CTA) 7.4 µs per
+    // iteration against 7.6 as a grid, 96² 8.5 against 7.4
+    if (chunks > kStripThreads / 32) return false;
+    if (at > kStripSmem || S.cluster * std::max(tasks, chunks) >= 65535 || S.units > 256 || S.vec_blocks > 256) return false;
+    S.bytes = (int)at;
+    S.max_tasks = (int)tasks;
+    S.max_chunks = (int)chunks;
+    S.max_nl = (int)nl;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(S.cluster);
+    cfg.blockDim = dim3(kStripThreads);
+    cfg.dynamicSmemBytes = S.bytes;
+    cfg.stream = H.stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = S.cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int fits = 0;
+    if (cudaFuncSetAttribute(k_cg64_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, kStripSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(k_cg64_strip, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&fits, (const void*)k_cg64_strip, &cfg) != cudaSuccess || fits < 1) {
+        cudaGetLastError();
+        return false;
+    }
+    GG_CUDA(cudaLaunchKernelEx(&cfg, k_cg64_strip, A, S));
+    return true;
 }
 
 template <int DIM>
 int run(Handle& H, Cg64Args& A) {
+    if (DIM == 2 && run_strip(H, A)) return 0;
     constexpr int T = cg64_threads<DIM>(), per = T / 256;
     const int work = std::max(A.tiles << DIM, A.vec_blocks);
-    const void* fc = (const void*)k_cg64<DIM, true>;
-    const void* fg = (const void*)k_cg64<DIM, false>;
-    // one cluster while every tile and vector block finds a group of its own in it: 16² / 32² /
-    // 48² took 5.9 / 5.2 / 5.5 µs per iteration against 7.4 / 7.0 / 7.6 as a grid; with a
-    // second round the 16 SMs lose to the grid (72²: 9.4 against 7.6 µs)
-    if (work <= kCluster * per && cluster_fits(fc, T) > 0) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(kCluster);
-        cfg.blockDim = dim3(T);
-        cfg.stream = H.stream;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = kCluster;
-        at.val.clusterDim.y = at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        GG_CUDA(cudaLaunchKernelEx(&cfg, k_cg64<DIM, true>, A));
-        return 0;
-    }
+    const void* fn = (const void*)k_cg64<DIM>;
     int per_sm = 0;
-    GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fg, T, 0));
+    GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, 0));
     if (per_sm < 1) return 1;
     const int grid = std::min((work + per - 1) / per, per_sm * num_sms());
     GG_CUDA(cudaMemsetAsync(A.gb, 0, sizeof(GridBarrier), H.stream));
     void* args[] = {(void*)&A};
-    GG_CUDA(cudaLaunchCooperativeKernel(fg, dim3(grid), dim3(T), args, 0, H.stream));
+    GG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(T), args, 0, H.stream));
     return 0;
 }
 

@@ -11,11 +11,12 @@ from gale_b200.stokes import (BodyForce, MaterialViscosity, Mesh, RheologyMateri
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [(2, 2), (3, 2), (33, 5), (31, 17), (64, 33), (65, 63), (2, 2, 2), (5, 3, 2), (33, 4, 3),
+@pytest.mark.parametrize("n", [(2, 2), (1, 1), (3, 2), (33, 5), (100, 3), (5, 90), (31, 17), (64, 33), (64, 64), (65, 63), (75, 70), (2, 2, 2), (5, 3, 2), (33, 4, 3),
                                (12, 11, 9)],
                          ids=lambda n: "x".join(map(str, n)))
 def test_cg64_against_oracle(oracle_mod, n):
-    """Partial tiles, single rows, one vector block, one cluster and a grid of CTAs."""
+    """Partial tiles, single rows, one vector block, strips of one to several row pairs in a
+    cluster of 1 to 16 CTAs, and a grid of CTAs."""
     dim = len(n)
     rng = np.random.default_rng(sum(n))
     mesh = Mesh(dim, n)
