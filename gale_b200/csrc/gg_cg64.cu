@@ -235,8 +235,9 @@ __global__ void __launch_bounds__(cg64_threads<DIM>(), 1) k_cg64(const __grid_co
                 for (int c = 0; c < DIM; c++)
 #pragma unroll
                     for (int a = 0; a < NS; a++) m[c][a] = zz[c][a] + beta * pp[c][a];
-                en[0] = element_compute<DIM, double, true>(mk, m, M, -1, [&](int c, int a, double v) {
-                    __stcg(A.ye + q.term + (int64_t)(a * DIM + c) * A.class_max, v);
+                en[0] = element_compute<DIM, double, true>(mk, m, M, -1, [&](int c, int row, double v0, double v1) {
+                    __stcg(A.ye + q.term + (int64_t)(2 * row * DIM + c) * A.class_max, v0);
+                    __stcg(A.ye + q.term + (int64_t)((2 * row + 1) * DIM + c) * A.class_max, v1);
                 });
             }
             group_sum<1>(en, g);
@@ -635,8 +636,9 @@ k_cg64_strip(const __grid_constant__ Cg64Args A, const __grid_constant__ Cg64Str
                 for (int c = 0; c < 2; c++)
 #pragma unroll
                     for (int a = 0; a < NS; a++) m[c][a] = zz[c][a] + beta * pp[c][a];
-                en = element_compute<2, double, true>(mk, m, M, -1, [&](int c, int a, double v) {
-                    cluster_store(taddr[(a * 2 + c) * te_n + te], v);
+                en = element_compute<2, double, true>(mk, m, M, -1, [&](int c, int row, double v0, double v1) {
+                    cluster_store(taddr[(4 * row + c) * te_n + te], v0);
+                    cluster_store(taddr[(4 * row + 2 + c) * te_n + te], v1);
                 });
             }
 #pragma unroll

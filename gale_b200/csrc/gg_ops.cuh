@@ -61,12 +61,13 @@ __device__ __forceinline__ int32_t local_node(int32_t n0, int32_t nn0, int32_t n
 // (corner a = (dx, dy, dz) bits) and moments M; `fixed` holds bit 8q + 4dx + c for the
 // Dirichlet components of the corners of row q.  Shared by every loader of the apply.
 // c_only ≥ 0 forms and scatters output component c_only alone (the transform and the
-// velocity gradients still use every component).  emit(c, a, v) takes the element's term
-// of component c at corner a.
+// velocity gradients still use every component).  emit(c, q, v0, v1) takes the element's
+// terms of component c at the corners 2q and 2q + 1 (neighbours along x).
 template <int DIM, typename R, bool kEnergy, class Emit>
 __device__ __forceinline__ double element_compute(const MeshK& mk, R (&m)[DIM][1 << DIM],
                                                   const R (&M)[n_moments<DIM>()], int c_only, Emit emit) {
     constexpr int NS = 1 << DIM;
+    constexpr int NR = NS / 2;
     R kap[DIM];
 #pragma unroll
     for (int d = 0; d < DIM; d++) kap[d] = (R)mk.kappa[d];
@@ -138,7 +139,7 @@ __device__ __forceinline__ double element_compute(const MeshK& mk, R (&m)[DIM][1
                     Q[a | (1 << d)] = q0 + q1;
                 }
 #pragma unroll
-        for (int a = 0; a < NS; a++) emit(c, a, Q[a]);
+        for (int q = 0; q < NR; q++) emit(c, q, Q[2 * q], Q[2 * q + 1]);
     }
     return energy;
 }
@@ -153,9 +154,10 @@ __device__ __forceinline__ double element_compute_scatter(const MeshK& mk, R (&m
     int32_t rowoff[NR];
 #pragma unroll
     for (int q = 0; q < NR; q++) rowoff[q] = (q & 1) * nn0 + (DIM == 3 ? ((q >> 1) & 1) * nn01 : 0);
-    return element_compute<DIM, R, kEnergy>(mk, m, M, c_only, [&](int c, int a, R v) {
-        const int q = a >> 1;
-        if (!((fixed >> (8 * q + 4 * (a & 1) + c)) & 1)) atomicAdd(y + c * nnode + n0 + rowoff[q] + (a & 1), v);
+    return element_compute<DIM, R, kEnergy>(mk, m, M, c_only, [&](int c, int q, R v0, R v1) {
+        R* yr = y + c * nnode + n0 + rowoff[q];
+        if (!((fixed >> (8 * q + c)) & 1)) atomicAdd(yr, v0);
+        if (!((fixed >> (8 * q + 4 + c)) & 1)) atomicAdd(yr + 1, v1);
     });
 }
 
