@@ -10,12 +10,21 @@
 // 9.8 ms, the cells 1.1 ms; 14 threads gained nothing on either (a transfer then waits for
 // the last of them to wake).
 //
-// The slots (kWorkers · 2 · kSlot = 32 MB of pinned memory per device) and the threads are
+// The slots (kWorkers · 2 · kSlot = 16 MB of pinned memory per device) and the threads are
 // shared by the process, made by the first large transfer and given back when the last handle is
 // destroyed.  One transfer uses them at a time; one that finds them busy (another thread's
 // handle) takes the plain copy, so no caller waits for another.
+//
+// A program that keeps one handle at a time pays for the slots with each, so they have to
+// be cheap: pinned pages of 4 KB cost 12-25 ms for 32 MB (cudaMallocHost) and 3-11 ms to
+// give back, huge pages registered in place 3-4 and 0.8 ms for 16 MB.  Slots of 0.25 / 0.5 /
+// 1 / 2 MB moved the cells in 1.8 / 1.5 / 1.3 / 1.3 ms and the coordinates in 13.5 / 11.4 /
+// 9.5 / 10.4 ms, device work included.
+#include <sys/mman.h>
+
 #include <algorithm>
 #include <condition_variable>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -30,7 +39,10 @@ namespace gg {
 namespace {
 
 constexpr int kWorkers = 8;
-constexpr size_t kSlot = size_t(2) << 20;
+constexpr size_t kSlot = size_t(1) << 20;
+constexpr size_t kHugePage = size_t(2) << 20;
+constexpr size_t kSlots = kSlot * 2 * kWorkers;
+static_assert(kSlots % kHugePage == 0, "the slots are whole huge pages");
 constexpr size_t kMinChunk = size_t(128) << 10;
 constexpr size_t kMinOut = size_t(1) << 20;   // to the host: the page faults alone pay for the threads
 constexpr size_t kMinIn = size_t(12) << 20;   // to the device: the driver stages 3-10 MB as fast (0.34-1.06 ms), 21 MB in 2.2 ms against 1.7
@@ -46,6 +58,7 @@ struct Job {
 // The slots, their events and the threads of one device.
 struct Stager {
     int dev;
+    void* map = MAP_FAILED;  // the slots, with room to align them
     char* slots = nullptr;
     cudaEvent_t ev[kWorkers][2] = {};
     std::vector<std::thread> threads;
@@ -60,7 +73,12 @@ struct Stager {
     explicit Stager(int d) : dev(d) {}
 
     bool start() {
-        if (cudaMallocHost(&slots, kSlot * 2 * kWorkers) != cudaSuccess) {
+        map = mmap(nullptr, kSlots + kHugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        if (map == MAP_FAILED) return false;
+        const uintptr_t up = (reinterpret_cast<uintptr_t>(map) + kHugePage - 1) & ~(uintptr_t)(kHugePage - 1);
+        slots = reinterpret_cast<char*>(up);
+        madvise(slots, kSlots, MADV_HUGEPAGE);  // refused: pages of 4 KB, which only cost time
+        if (cudaHostRegister(slots, kSlots, cudaHostRegisterPortable) != cudaSuccess) {
             cudaGetLastError();
             slots = nullptr;
             return false;
@@ -89,7 +107,8 @@ struct Stager {
         for (auto& e : ev)
             for (auto& x : e)
                 if (x) cudaEventDestroy(x);
-        if (slots) cudaFreeHost(slots);
+        if (slots) cudaHostUnregister(slots);
+        if (map != MAP_FAILED) munmap(map, kSlots + kHugePage);
     }
 
     void loop(int w) {
