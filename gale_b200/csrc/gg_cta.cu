@@ -14,10 +14,11 @@
 //                     step for step, FP64, Ĝ-preconditioned, as gg_solve.cu:uzawa_solve;
 //   inner solves      FP64 defect correction around FP32 flexible-CG sweeps preconditioned
 //                     by a Chebyshev–Jacobi V-cycle, the stopping rules of inner_solve;
-//   element applies   the matrix-free kernel of gg_ops.cuh over the element parity classes
-//                     with a block barrier between classes: no two threads add into the same
-//                     node at once, and every node sums its element terms in class order, so
-//                     a problem solved here gives the same bits on every run.
+//   element applies   the matrix-free arithmetic of gg_ops.cuh; every node sums its element
+//                     terms in the order of the element parity classes, so a problem solved
+//                     here gives the same bits on every run: 2D FP32 applies store the terms
+//                     and gather them per node (cta_apply2), 3D and FP64 ones add class by
+//                     class with a block barrier between (cta_apply).
 // Vectors live in global memory (L2-resident for these sizes); inside the launch they are
 // read with L1-cached loads, coherent within the CTA across its block barriers.
 #include <math.h>
@@ -69,6 +70,7 @@ struct CtaProblem {
     const double* hvec;
     double *u, *vstar, *ftmp, *q, *qtmp, *r, *s, *bb, *r64;
     float *r32, *z32, *p32, *Ap32, *e32;
+    float* terms;  // 2D: element terms of an FP32 apply, [8][elements]
     float* lam;            // [kCtaMaxLevels] λ_max per level (written here)
     gg_uzawa_stats* stats;  // device copy of the problem's statistics
     int32_t* status;
@@ -132,6 +134,107 @@ __device__ __noinline__ double cta_apply(const MeshK& mk, const R* mom, const ui
         __syncthreads();
     }
     return en;
+}
+
+// One element's nodal values and moments (the gather of element_apply_scatter).
+__device__ __forceinline__ void cta_gather2(const MeshK& mk, const float* __restrict__ mom, const float* x, int e, int i,
+                                            int j, float (&m)[2][4], float (&M)[6]) {
+    const int nn0 = mk.nn[0], nel = (int)mk.nel;
+    const float* xr = x + i + nn0 * j;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const float* at = xr + c * (int)mk.nnode + q * nn0;
+            m[c][2 * q] = ldg_cg(at);
+            m[c][2 * q + 1] = ldg_cg(at + 1);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 6; q++) M[q] = mom[e + q * nel];
+}
+
+// y = K x in 2D from element terms: every element stores its eight corner terms
+// (terms[4c + corner][element]), and after one barrier every node adds the terms of its four
+// elements in class order — the sums cta_apply forms, without its barrier per class, its
+// reductions to L2 and its half-used sectors (a class has every second element of a row).
+// What bounds the solve is the latency of these passes on one SM, 16 warps with a few loads
+// each: four class passes cost a small level four barriers and four nearly empty rounds.
+// ms per problem, classes / terms: 16² 8.6 / 6.3, 32² 29.8 / 25.4, 48² 93 / 76, 64² 84 / 78,
+// 96² 246 / 225, 128² 361 / 349 (its terms, 512 KB, go through L2); 148 problems of up to 48²
+// 294 / 239.
+template <bool kEnergy>
+__device__ __noinline__ double cta_apply2(const MeshK& mk, const float* __restrict__ mom, const uint8_t* __restrict__ bc,
+                                          const float* x, float* y, float* terms) {
+    const int nel = (int)mk.nel, nnode = (int)mk.nnode, n0 = mk.n[0], n1 = mk.n[1], nn0 = mk.nn[0];
+    double en = 0.0;
+    if constexpr (kEnergy) {  // a thread's elements in cta_apply's order: its sum of energies is kept
+        for (int color = 0; color < 4; color++) {
+            const int px = color & 1, py = color >> 1;
+            const int c0 = (n0 - px + 1) >> 1, ncls = c0 * ((n1 - py + 1) >> 1);
+            for (int idx = threadIdx.x; idx < ncls; idx += blockDim.x) {
+                const int i = 2 * (idx % c0) + px, j = 2 * (idx / c0) + py, e = i + n0 * j;
+                float m[2][4], M[6];
+                cta_gather2(mk, mom, x, e, i, j, m, M);
+                en += element_compute<2, float, true>(mk, m, M, -1, [&](int c, int q, float v0, float v1) {
+                    terms[(4 * c + 2 * q) * nel + e] = v0;
+                    terms[(4 * c + 2 * q + 1) * nel + e] = v1;
+                });
+            }
+        }
+    } else {
+        for (int e0 = threadIdx.x; e0 < nel; e0 += 2 * blockDim.x) {  // two elements' loads in flight
+            const int e1 = e0 + blockDim.x;
+            const bool two = e1 < nel;
+            float ma[2][4], Ma[6], mb[2][4], Mb[6];
+            cta_gather2(mk, mom, x, e0, e0 % n0, e0 / n0, ma, Ma);
+            const int es = two ? e1 : e0;
+            cta_gather2(mk, mom, x, es, es % n0, es / n0, mb, Mb);
+            element_compute<2, float, false>(mk, ma, Ma, -1, [&](int c, int q, float v0, float v1) {
+                terms[(4 * c + 2 * q) * nel + e0] = v0;
+                terms[(4 * c + 2 * q + 1) * nel + e0] = v1;
+            });
+            if (two)
+                element_compute<2, float, false>(mk, mb, Mb, -1, [&](int c, int q, float v0, float v1) {
+                    terms[(4 * c + 2 * q) * nel + e1] = v0;
+                    terms[(4 * c + 2 * q + 1) * nel + e1] = v1;
+                });
+        }
+    }
+    __syncthreads();
+    for (int n = threadIdx.x; n < nnode; n += blockDim.x) {
+        const int i = n % nn0, j = n / nn0;
+        const uint32_t fixed = bc[n];
+        // the elements of even index come first along each axis
+        float v[2][4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int dx = (i & 1) ^ (k & 1), dy = (j & 1) ^ (k >> 1);
+            const int ei = i - dx, ej = j - dy;
+            const bool in = ei >= 0 && ei < n0 && ej >= 0 && ej < n1;
+            const float* at = terms + (dx + 2 * dy) * nel + (in ? ei + n0 * ej : 0);
+            v[0][k] = in ? ldg_cg(at) : 0.f;
+            v[1][k] = in ? ldg_cg(at + 4 * nel) : 0.f;
+        }
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            float sum = 0.f;
+#pragma unroll
+            for (int k = 0; k < 4; k++) sum += v[c][k];
+            y[n + c * nnode] = (fixed >> c) & 1 ? 0.f : sum;
+        }
+    }
+    __syncthreads();
+    return en;
+}
+
+// y = K x in FP32 (y zero on entry)
+template <int DIM, bool kEnergy>
+__device__ __forceinline__ double cta_apply32(const CtaLevel& L, const float* x, float* y, float* terms) {
+    if constexpr (DIM == 2)
+        return cta_apply2<kEnergy>(L.mk, L.mom32, L.bc, x, y, terms);
+    else
+        return cta_apply<DIM, float, kEnergy>(L.mk, L.mom32, L.bc, x, y);
 }
 
 template <typename R>
@@ -311,7 +414,7 @@ __device__ void cta_invert_diag(int64_t n, int64_t nnode, const uint8_t* bc, con
 
 // λ_max(D⁻¹A) by power steps from a hashed start (k_hash_fill, k_power_step, k_power_norm)
 template <int DIM>
-__device__ __noinline__ float cta_power(const CtaLevel& L) {
+__device__ __noinline__ float cta_power(const CtaLevel& L, float* terms) {
     const int64_t n = (int64_t)DIM * L.mk.nnode;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
         uint32_t h = (uint32_t)i * 2654435761u + 0x9e3779b9u;
@@ -324,7 +427,7 @@ __device__ __noinline__ float cta_power(const CtaLevel& L) {
     __syncthreads();
     double lam = 1.0;
     for (int step = 0; step < kCtaPowerSteps; step++) {
-        cta_apply<DIM, float, false>(L.mk, L.mom32, L.bc, L.x, L.t);
+        cta_apply32<DIM, false>(L, L.x, L.t, terms);
         double yy = 0.0, xx = 0.0;
         for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
             const float v = L.invd[i] * ldg_cg(&L.t[i]);
@@ -577,10 +680,10 @@ __device__ __noinline__ void cta_vcycle(const CtaProblem& P, const CtaCheb* cheb
         const int dl = l == 0 ? P.degree : min(P.degree, 2);
         cta_cheb_start(L, n, bl, xl, cheb[l].inv_theta);
         for (int k = 1; k < dl; k++) {
-            cta_apply<DIM, float, false>(L.mk, L.mom32, L.bc, L.d, L.t);
+            cta_apply32<DIM, false>(L, L.d, L.t, P.terms);
             cta_cheb_step(L, n, xl, cheb[l].c1[k], cheb[l].c2[k]);
         }
-        cta_apply<DIM, float, false>(L.mk, L.mom32, L.bc, L.d, L.t);
+        cta_apply32<DIM, false>(L, L.d, L.t, P.terms);
         cta_restrict<DIM>(L, P.lv[l + 1]);
     }
     {
@@ -596,7 +699,7 @@ __device__ __noinline__ void cta_vcycle(const CtaProblem& P, const CtaCheb* cheb
         } else {  // a long Chebyshev sweep from zero
             cta_cheb_start(C, n, C.b, C.x, cheb[ns].inv_theta);
             for (int k = 1; k < kCtaCoarseChebDegree; k++) {
-                cta_apply<DIM, float, false>(C.mk, C.mom32, C.bc, C.d, C.t);
+                cta_apply32<DIM, false>(C, C.d, C.t, P.terms);
                 cta_cheb_step(C, n, C.x, cheb[ns].c1[k], cheb[ns].c2[k]);
             }
         }
@@ -608,10 +711,10 @@ __device__ __noinline__ void cta_vcycle(const CtaProblem& P, const CtaCheb* cheb
         float* xl = l == 0 ? x0 : L.x;
         const int dl = l == 0 ? P.degree : min(P.degree, 2);
         cta_prolong<DIM>(L, xl, P.lv[l + 1]);
-        cta_apply<DIM, float, false>(L.mk, L.mom32, L.bc, xl, L.t);
+        cta_apply32<DIM, false>(L, xl, L.t, P.terms);
         cta_cheb_restart(L, n, bl, xl, cheb[l].inv_theta);
         for (int k = 1; k < dl; k++) {
-            cta_apply<DIM, float, false>(L.mk, L.mom32, L.bc, L.d, L.t);
+            cta_apply32<DIM, false>(L, L.d, L.t, P.terms);
             cta_cheb_step(L, n, xl, cheb[l].c1[k], cheb[l].c2[k]);
         }
     }
@@ -660,7 +763,7 @@ __device__ __noinline__ int cta_fcg(const CtaProblem& P, const CtaCheb* cheb, co
             Ap[i] = 0.f;
         }
         __syncthreads();
-        pAp = cta_sum(cta_apply<DIM, float, true>(mk, L0.mom32, L0.bc, p, Ap));
+        pAp = cta_sum(cta_apply32<DIM, true>(L0, p, Ap, P.terms));
         if (!(pAp > 0.0) || isinf(pAp)) return 2;
         const float alpha = (float)(rz / pAp);
         double rr = 0.0;
@@ -795,7 +898,7 @@ __device__ __noinline__ void cta_solve_problem(const CtaProblem& P, const CtaPar
     for (int l = 0; l < nl; l++) {
         const bool coarsest = l == nl - 1;
         if (coarsest && P.dense_n) break;
-        const float lam = cta_power<DIM>(P.lv[l]);
+        const float lam = cta_power<DIM>(P.lv[l], P.terms);
         if (threadIdx.x == 0) {
             const int deg = coarsest ? kCtaCoarseChebDegree : (l == 0 ? P.degree : min(P.degree, 2));
             s_cheb[l] = cta_cheb(lam, deg);
@@ -1096,6 +1199,10 @@ int cta_batch_solve(std::vector<Handle*>& hs, const gg_uzawa_params& prm, double
         P.p32 = H.p32.as<float>();
         P.Ap32 = H.Ap32.as<float>();
         P.e32 = H.e32.as<float>();
+        if (dim == 2) {
+            H.cg_terms.ensure(sizeof(float) * 8 * ne);
+            P.terms = H.cg_terms.as<float>();
+        }
         P.lam = H.cta_lam.as<float>();
         if (prm.reuse_pressure)
             GG_CUDA(cudaMemcpyAsync(H.q.p, p_out[i], sizeof(double) * ne, cudaMemcpyHostToDevice, H.stream));

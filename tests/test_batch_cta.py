@@ -8,11 +8,13 @@ batch, one CTA per problem (needs a B200).
   solving the same batch twice gives the same bits;
 - the batch reports one kernel launch per problem (the shared launch).
 """
+from dataclasses import replace
+
 import numpy as np
 import pytest
 
 from gale_b200 import workloads
-from gale_b200.stokes import StokesProblem, UzawaSolver
+from gale_b200.stokes import Mesh, StokesProblem, UzawaSolver
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +56,24 @@ def test_cta_batch_of_an_odd_count():
     for (ua, pa, sa), (ub, pb, sb) in zip(three, four):
         assert np.array_equal(ua, ub) and np.array_equal(pa, pb)
         assert sa["outer_iterations"] == sb["outer_iterations"] > 0
+
+
+@pytest.mark.parametrize("nx,ny", [(16, 32), (22, 24), (64, 8), (34, 30), (40, 26)])
+def test_cta_batch_of_ragged_2d_meshes(oracle_mod, nx, ny):
+    """Element counts around the block size and twice it (512, 528, 1020 and 1040 elements on
+    512 threads), uneven axes and odd coarse levels: as close to the converged solution as
+    the FP64 oracle at the same tolerance."""
+    mesh = Mesh(2, (nx, ny), (0.0, 0.0), (1.0, 1.0))
+    x = workloads.random_points(mesh, 12, np.random.default_rng(17))
+    inside = (x[:, 0] - 0.5) ** 2 + (x[:, 1] - 0.6) ** 2 < 0.04
+    w = replace(workloads.sinker_2d(n=4), mesh=mesh, coords=x, material=inside.astype(np.int32))
+    (u, p, _), = StokesProblem.solve_batch([w.apply(StokesProblem(mesh))],
+                                           UzawaSolver(tolerance=1e-6, precision="mixed", inner="mg"))
+    O = w.apply(oracle_mod.OracleProblem(mesh))
+    O.assemble()
+    ut, pt, _ = O.uzawa(UzawaSolver(tolerance=1e-11, innerRtolFactor=0.01, maxIterations=5000,
+                                    innerMaxIterations=200000))
+    uo, po, _ = O.uzawa(UzawaSolver(tolerance=1e-6))
+    pc, ptc, poc = p - p.mean(), pt - pt.mean(), po - po.mean()
+    assert rel(u, ut) <= 1.5 * rel(uo, ut) + 1e-6
+    assert rel(pc, ptc) <= 1.5 * rel(poc, ptc) + 1e-6
