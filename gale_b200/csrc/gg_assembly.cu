@@ -221,7 +221,7 @@ __device__ PointOut run_rheologies(const MeshK& mk, const gg_material& m, const 
 }
 
 // Per point: viscosity in FP64, with kBoth also by the FP32 rheology chain, and the
-// temperature where a force term reads it (temp null: none does).
+// temperature where a force term reads it (temp null: none does; T null: it is 0).
 // Bound by its loads and stores (60-90 bytes per point) once enough warps cover the
 // exponential's latency: at 255 registers, one block per SM, it took 651 µs for 7.1 M points;
 // three blocks spill a little in the yield laws and take 232 (two took 3 % more), 32-bit element
@@ -255,7 +255,7 @@ k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const double*
         }
         if (temp) {
             double Tp = 0.0;
-            if (rayleigh != 0.0 || m.alpha != 0.0) {
+            if (T && (rayleigh != 0.0 || m.alpha != 0.0)) {
                 double N[NEN];
                 shape<DIM, double>(xi, N);
 #pragma unroll
@@ -479,12 +479,13 @@ static void gather_corners(Handle& H, R* kdiag, double* f) {
     GG_CUDA(cudaGetLastError());
 }
 
-// Whether the force weights of a build can be anything but zero: a zero gravity or Rayleigh
-// number makes them zero unless a factor beside it is not finite (a density, or through a
-// thermal expansivity the temperature).
+// Whether the force weights of a build can be anything but zero.  A zero gravity or Rayleigh
+// number, or a temperature that is not set (0), makes them zero unless the factor beside it is
+// not finite: a density, a thermal expansivity (through it the temperature) or the Rayleigh
+// number.  Those weights are NaN, and so are the force and the solve that reads it.
 static bool any_alpha(const Handle& H) {
     for (const gg_material& m : H.materials)
-        if (H.has_T && m.alpha != 0.0) return true;
+        if (H.has_T ? m.alpha != 0.0 : !std::isfinite(m.alpha)) return true;
     return false;
 }
 static bool phi_nonzero(const Handle& H) {
@@ -493,7 +494,9 @@ static bool phi_nonzero(const Handle& H) {
         if (!std::isfinite(m.density)) return true;
     return false;
 }
-static bool psi_nonzero(const Handle& H) { return H.has_T && (H.force.rayleigh != 0.0 || any_alpha(H)); }
+static bool psi_nonzero(const Handle& H) {
+    return !std::isfinite(H.force.rayleigh) || (H.has_T && (H.force.rayleigh != 0.0 || any_alpha(H)));
+}
 
 template <int DIM>
 static void launch_build(Handle& H, bool mixed, int prev, const double* pu, const double* pp) {

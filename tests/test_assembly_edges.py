@@ -55,3 +55,25 @@ def test_build_against_oracle(oracle_mod, n, most, dvc):
     y = O.apply_K(v)
     assert rel(G.apply_K(v), y) <= 1e-12
     assert rel(G.apply_K(v, "mixed"), y) <= 1e-5
+
+
+@pytest.mark.parametrize("T", [None, 0.0], ids=["no T", "T=0"])
+@pytest.mark.parametrize("gravity,ra,alpha,density", [(1.0, np.inf, 0.0, 1.0), (1.0, np.nan, 0.0, 1.0),
+                                                      (0.0, 0.0, np.inf, 1.0), (0.0, 0.0, 0.0, np.nan)], ids=str)
+def test_nonfinite_force_terms_stay_nonfinite(T, gravity, ra, alpha, density):
+    """A weight that is zero times a factor that is not finite is NaN, with and without a
+    temperature: an invalid body force is not taken for a zero one."""
+    mesh = Mesh(2, (3, 4))
+    G = StokesProblem(mesh)
+    G.set_velocity_bc(free_slip(2))
+    G.set_materials([RheologyMaterial([MaterialViscosity(1.0)], density=density, alpha=alpha)])
+    G.set_body_force(BodyForce(gravity=gravity, rayleighNumber=ra))
+    if T is not None:
+        G.set_temperature(np.full(G.nnode, T))
+    G.set_points(workloads.random_points(mesh, 5, np.random.default_rng(0)))
+    G.locate()
+    G.build_operator("fp64")
+    f = G.rhs()[0].reshape(G.nnode, 2)
+    # the free vertical components of the inner rows of nodes
+    inner = np.arange(G.nnode).reshape(5, 4)[1:-1].ravel()
+    assert np.isnan(f[inner, 1]).all()
