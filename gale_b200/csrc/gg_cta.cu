@@ -689,18 +689,21 @@ __device__ __noinline__ void cta_vcycle(const CtaProblem& P, const CtaCheb* cheb
     {
         const CtaLevel& C = P.lv[ns];
         const int64_t n = (int64_t)DIM * C.mk.nnode;
+        // a mesh that does not coarsen (an odd axis, or few dofs) has the fine level here
+        const float* bc = ns == 0 ? b0 : C.b;
+        float* xc = ns == 0 ? x0 : C.x;
         if (P.dense_n) {  // x = A⁻¹ b, one thread per row
             for (int64_t row = threadIdx.x; row < n; row += blockDim.x) {
                 float s = 0.f;
-                for (int64_t k = 0; k < n; k++) s += dense[row * n + k] * ldg_cg(&C.b[k]);
-                C.x[row] = s;
+                for (int64_t k = 0; k < n; k++) s += dense[row * n + k] * ldg_cg(&bc[k]);
+                xc[row] = s;
             }
             __syncthreads();
         } else {  // a long Chebyshev sweep from zero
-            cta_cheb_start(C, n, C.b, C.x, cheb[ns].inv_theta);
+            cta_cheb_start(C, n, bc, xc, cheb[ns].inv_theta);
             for (int k = 1; k < kCtaCoarseChebDegree; k++) {
                 cta_apply32<DIM, false>(C, C.d, C.t, P.terms);
-                cta_cheb_step(C, n, C.x, cheb[ns].c1[k], cheb[ns].c2[k]);
+                cta_cheb_step(C, n, xc, cheb[ns].c1[k], cheb[ns].c2[k]);
             }
         }
     }
@@ -1098,8 +1101,8 @@ bool cta_batch_supported(const gg_uzawa_params& prm) {
 }
 
 // Levels of a problem for the CTA solver: halve while every axis is even and ≥ 4 elements
-// and the level has more than kCtaDenseMax dofs; the coarsest is inverted densely when it
-// has at most kCtaDenseMax dofs.
+// and the level has more than kCtaDenseMax dofs; the coarsest (the fine level itself, where
+// none of that holds) is inverted densely when it has at most kCtaDenseMax dofs.
 static void cta_levels(Handle& H, std::vector<MeshK>& mks, int& dense_n) {
     mks.clear();
     mks.push_back(H.mk);
@@ -1120,7 +1123,7 @@ static void cta_levels(Handle& H, std::vector<MeshK>& mks, int& dense_n) {
         mks.push_back(make_mesh(cd));
     }
     const int64_t nc = (int64_t)H.dim * mks.back().nnode;
-    dense_n = (mks.size() > 1 && nc <= kCtaDenseMax) ? (int)nc : 0;
+    dense_n = nc <= kCtaDenseMax ? (int)nc : 0;
 }
 
 // Solve every problem (located and built with the FP32 moments) in one launch.  status[i]

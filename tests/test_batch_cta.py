@@ -77,3 +77,28 @@ def test_cta_batch_of_ragged_2d_meshes(oracle_mod, nx, ny):
     pc, ptc, poc = p - p.mean(), pt - pt.mean(), po - po.mean()
     assert rel(u, ut) <= 1.5 * rel(uo, ut) + 1e-6
     assert rel(pc, ptc) <= 1.5 * rel(poc, ptc) + 1e-6
+
+
+@pytest.mark.parametrize("n", [(8, 8), (9, 7), (4, 3), (27, 19), (31, 33), (5, 4, 3), (9, 7, 5)],
+                         ids=lambda n: "x".join(map(str, n)))
+def test_cta_batch_of_meshes_that_do_not_coarsen(oracle_mod, n):
+    """One multigrid level: an odd axis, or few enough dofs.  As close to the converged
+    solution as the FP64 oracle at the same tolerance."""
+    dim = len(n)
+    mesh = Mesh(dim, n)
+    w = workloads.sinker_2d(n=4) if dim == 2 else workloads.creep_3d(n=4)
+    x = workloads.random_points(mesh, 12, np.random.default_rng(17))
+    inside = np.sum((x - 0.55) ** 2, 1) < 0.06
+    w = replace(w, mesh=mesh, coords=x, material=inside.astype(np.int32) if dim == 2 else np.zeros(len(x), np.int32),
+                temperature=None if dim == 2 else np.random.default_rng(3).random(int(np.prod(np.add(n, 1)))))
+    probs = [w.apply(StokesProblem(mesh)) for _ in range(2)]
+    (u, p, st), (u2, p2, _) = StokesProblem.solve_batch(probs, UzawaSolver(tolerance=1e-6, precision="mixed", inner="mg"))
+    assert st["rel_residual"] <= 1e-6 and np.array_equal(u, u2) and np.array_equal(p, p2)
+    O = w.apply(oracle_mod.OracleProblem(mesh))
+    O.assemble()
+    ut, pt, _ = O.uzawa(UzawaSolver(tolerance=1e-11, innerRtolFactor=0.01, maxIterations=5000,
+                                    innerMaxIterations=200000))
+    uo, po, _ = O.uzawa(UzawaSolver(tolerance=1e-6))
+    pc, ptc, poc = p - p.mean(), pt - pt.mean(), po - po.mean()
+    assert rel(u, ut) <= 1.5 * rel(uo, ut) + 1e-6
+    assert rel(pc, ptc) <= 1.5 * rel(poc, ptc) + 1e-6
