@@ -857,8 +857,12 @@ void launch_group(const DvcArgs& a, DvcGroup f, int cap, cudaStream_t st) {
     f.mnx = (65536u + a.nx - 1) / a.nx;
     f.mny = (65536u + a.ny - 1) / a.ny;
     constexpr int per = kGroupThreads / G;
+    // At most 64 points, 1024 cells and a ring of 1024: below the shared memory a kernel may
+    // use without asking.  The limit is state of the function, shared by every host thread, so
+    // nothing sets it to the size of one launch.
+    static_assert(per * (8 * DIM * kGroupPts + kMaxCells / 8 + kMaxCells + 2 * 1024 + 7 * kGroupPts + 48) <= 48 * 1024 - 3 * 8 * kAxis,
+                  "a block of groups fits the default shared memory");
     const size_t smem = (size_t)f.stride * per;
-    GG_CUDA(cudaFuncSetAttribute(k_dvc_group<DIM, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_dvc_group<DIM, G><<<(unsigned)((a.nel + per - 1) / per), kGroupThreads, smem, st>>>(a, f);
     GG_CUDA(cudaGetLastError());
 }

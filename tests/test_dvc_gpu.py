@@ -1,6 +1,8 @@
 """DVCWeights and PCDVC on the GPU against the CPU oracle (needs a B200).  Same
 algorithm, same double roundings: the integration points, weights and the rebuilt point
 set must agree bit for bit; the moments built from them to summation order."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -130,3 +132,33 @@ def test_dvc_weights_uneven_elements(oracle_mod, dim, res, most):
         cent, w_ref = oracle_mod.dvc_cell(dim, res, local[idx])
         assert np.array_equal(wt[idx], w_ref)
         assert np.array_equal(xi[idx], cent)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_dvc_from_threads_of_different_density(dim):
+    """Handles of different grids and point counts take their diagrams at the same time (the
+    launches need different amounts of shared memory): every call succeeds, with the weights
+    the handle gives alone."""
+    def make(res, ppe):
+        mesh = Mesh(dim, [1] * dim)
+        x = workloads.random_points(mesh, ppe, np.random.default_rng(res))
+        G = StokesProblem(mesh)
+        G.set_points(x, np.zeros(len(x), dtype=np.int32))
+        G.set_weights("dvc", res)
+        G.locate()
+        return G, G.integration_points()[1]
+    probs = [make(*((4, 20) if k % 2 else (2, 1))) for k in range(16)]
+    refused = []
+
+    def work(G):
+        for _ in range(3000):
+            if G.lib.gg_locate(G.h, None) != 0:
+                refused.append(G.lib.gg_last_error(G.h).decode())
+    ts = [threading.Thread(target=work, args=(G,)) for G, _ in probs]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not refused, (len(refused), refused[0])
+    for G, w in probs:
+        assert np.array_equal(G.integration_points()[1], w)
