@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "gg_cluster_addr.h"
 #include "gg_grid.cuh"
 #include "gg_internal.cuh"
 #include "gg_kernels.cuh"
@@ -343,8 +344,6 @@ __global__ void __launch_bounds__(cg64_threads<DIM>(), 1) k_cg64(const __grid_co
 // one chunk of 32 vector entries, so the partial sums exchanged are those of the warps, and
 // they are added up in block_sum's order.
 constexpr int kStripThreads = 576;  // 18 warps of ≤ 112 registers: a 64² strip has 17-18 chunks
-constexpr unsigned kNoAddr = 0xffffffffu;
-constexpr unsigned kRemote = 0x80000000u;  // marks an address in another CTA (cluster addresses stay below)
 
 struct Cg64Strip {
     int cluster;
@@ -356,20 +355,22 @@ struct Cg64Strip {
 };
 
 __device__ __forceinline__ unsigned shared_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-// address of p in the cluster's CTA `rank`; in this CTA (`me`) the plain shared address, which
-// lies below the cluster window's per-CTA stride
+// address of p in the cluster's CTA `rank`, marked as remote; in this CTA (`me`) the plain
+// shared address
 __device__ __forceinline__ unsigned cluster_addr(const void* p, int rank, int me) {
     const unsigned a = shared_addr(p);
     unsigned r;
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return rank == me ? a : (r | kRemote);
+    return rank == me ? a : mark_remote(r);
 }
+// the mark comes off in the address offset
 __device__ __forceinline__ void cluster_store(unsigned a, double v) {
+    static_assert(kRemoteBit == 1u, "the offset of the remote store");
     asm volatile(
-        "{\n\t.reg .pred r;\n\t.reg .b32 t;\n\t"
-        "setp.lt.s32 r, %0, 0;\n\tand.b32 t, %0, 0x7fffffff;\n\t"
-        "@r st.shared::cluster.f64 [t], %1;\n\t@!r st.shared::cta.f64 [t], %1;\n\t}" ::"r"(a),
-        "d"(v)
+        "{\n\t.reg .pred r;\n\t"
+        "setp.ne.u32 r, %1, 0;\n\t"
+        "@r st.shared::cluster.f64 [%0+-1], %2;\n\t@!r st.shared::cta.f64 [%0], %2;\n\t}" ::"r"(a),
+        "r"(a & kRemoteBit), "d"(v)
         : "memory");
 }
 __device__ __forceinline__ void cluster_barrier() {
