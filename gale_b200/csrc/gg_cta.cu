@@ -105,7 +105,9 @@ __device__ __noinline__ double cta_sum(double v) {
 
 // Vectors written inside the launch are read with plain (L1-cached) loads: every value a
 // thread reads was written by a thread of the same CTA before a block barrier, which makes
-// it visible in L1; no read-only (non-coherent) load touches them.
+// it visible in L1; no read-only (non-coherent) load touches them.  That holds for the coarse
+// levels' moments and masks too, so no pointer to them is both const and __restrict__ unless
+// its loads are spelled out (element_apply_scatter's kLoad 2).
 template <typename T>
 __device__ __forceinline__ T ldg_cg(const T* p) { return __ldca(p); }
 
@@ -137,7 +139,7 @@ __device__ __noinline__ double cta_apply(const MeshK& mk, const R* mom, const ui
 }
 
 // One element's nodal values and moments (the gather of element_apply_scatter).
-__device__ __forceinline__ void cta_gather2(const MeshK& mk, const float* __restrict__ mom, const float* x, int e, int i,
+__device__ __forceinline__ void cta_gather2(const MeshK& mk, const float* mom, const float* x, int e, int i,
                                             int j, float (&m)[2][4], float (&M)[6]) {
     const int nn0 = mk.nn[0], nel = (int)mk.nel;
     const float* xr = x + i + nn0 * j;
@@ -151,7 +153,7 @@ __device__ __forceinline__ void cta_gather2(const MeshK& mk, const float* __rest
         }
     }
 #pragma unroll
-    for (int q = 0; q < 6; q++) M[q] = mom[e + q * nel];
+    for (int q = 0; q < 6; q++) M[q] = ldg_cg(mom + e + q * nel);
 }
 
 // y = K x in 2D from element terms: every element stores its eight corner terms
@@ -164,7 +166,7 @@ __device__ __forceinline__ void cta_gather2(const MeshK& mk, const float* __rest
 // 96² 246 / 225, 128² 361 / 349 (its terms, 512 KB, go through L2); 148 problems of up to 48²
 // 294 / 239.
 template <bool kEnergy>
-__device__ __noinline__ double cta_apply2(const MeshK& mk, const float* __restrict__ mom, const uint8_t* __restrict__ bc,
+__device__ __noinline__ double cta_apply2(const MeshK& mk, const float* mom, const uint8_t* bc,
                                           const float* x, float* y, float* terms) {
     const int nel = (int)mk.nel, nnode = (int)mk.nnode, n0 = mk.n[0], n1 = mk.n[1], nn0 = mk.nn[0];
     double en = 0.0;
@@ -204,7 +206,7 @@ __device__ __noinline__ double cta_apply2(const MeshK& mk, const float* __restri
     __syncthreads();
     for (int n = threadIdx.x; n < nnode; n += blockDim.x) {
         const int i = n % nn0, j = n / nn0;
-        const uint32_t fixed = bc[n];
+        const uint32_t fixed = ldg_cg(bc + n);
         // the elements of even index come first along each axis
         float v[2][4];
 #pragma unroll

@@ -161,6 +161,8 @@ __device__ __forceinline__ double element_compute_scatter(const MeshK& mk, R (&m
     });
 }
 
+// kLoad: how the operands are read.  0 plain; 1 x past L1 (written by other SMs in the same
+// launch); 2 everything through L1 (moments and mask too may have been written by this CTA).
 // kAxpy: the nodal values are x + beta·x2, formed at the gather (a flexible-CG direction
 // p = z + βp applied without storing it first; an FP64 iterate plus its FP32 correction).
 template <int DIM, typename R, int kLoad = 0, bool kEnergy = true, bool kAxpy = false, typename X2 = R>
@@ -184,7 +186,8 @@ __device__ __forceinline__ double element_apply_scatter(const MeshK& mk, const R
 #pragma unroll
     for (int q = 0; q < NR; q++) {
         const uint8_t* br = bcmask + n0 + rowoff[q];
-        fixed |= ((uint32_t)br[0] | ((uint32_t)br[1] << 4)) << (8 * q);
+        const uint32_t b0 = kLoad == 2 ? __ldca(br) : br[0], b1 = kLoad == 2 ? __ldca(br + 1) : br[1];
+        fixed |= (b0 | (b1 << 4)) << (8 * q);
     }
 
     R m[DIM][NS];
@@ -206,7 +209,7 @@ __device__ __forceinline__ double element_apply_scatter(const MeshK& mk, const R
     R M[NM];
     const R* Me = mom + e;
 #pragma unroll
-    for (int q = 0; q < NM; q++) M[q] = Me[q * nel];
+    for (int q = 0; q < NM; q++) M[q] = kLoad == 2 ? __ldca(Me + q * nel) : Me[q * nel];
     return element_compute_scatter<DIM, R, kEnergy>(mk, m, M, fixed, y, n0, c_only);
 }
 
