@@ -178,6 +178,7 @@ int gg_create(const gg_mesh_desc* mesh, gg_handle** out) {
         H.nnode = H.mk.nnode;
         H.ndof = H.nnode * H.dim;
         if (H.nel >= (int64_t)INT32_MAX) throw gg::CudaError(cudaErrorInvalidValue, "mesh too large", __FILE__, __LINE__);
+        GG_CUDA(cudaGetDevice(&H.device));
         GG_CUDA(cudaStreamCreateWithFlags(&H.stream, cudaStreamNonBlocking));
         GG_CUDA(cudaEventCreate(&H.ev0));
         GG_CUDA(cudaEventCreate(&H.ev1));

@@ -211,11 +211,12 @@ bool pageable(const void* host) {
     return a.type == cudaMemoryTypeUnregistered;
 }
 
-// false: not moved (small, pinned, busy or no slots)
+// false: not moved (small, pinned, busy or no slots, or the calling thread is on another
+// device than the handle: its events could not be recorded on the handle's stream)
 bool staged(Handle& H, void* host, void* device, size_t bytes, bool to_host) {
     if (bytes < (to_host ? kMinOut : kMinIn) || !pageable(host)) return false;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev != H.device || dev < 0 || dev >= kMaxDevices) return false;
     PerDevice& D = per_device(dev);
     std::unique_lock<std::mutex> lk(D.mu, std::try_to_lock);
     if (!lk.owns_lock()) return false;

@@ -67,6 +67,7 @@ struct Handle {
     MeshK mk{};
     int dim = 0, nm = 0;
     int64_t nel = 0, nnode = 0, ndof = 0;
+    int device = 0;  // the device the handle was made on
     cudaStream_t stream = nullptr;
     std::string err;
     std::string fail_where;  // stage at which the last Uzawa solve stopped early

@@ -1,0 +1,80 @@
+"""The host side of the staged transfers (gale_b200/csrc/gg_copy.cu) on the CPU: the file
+compiled for the host against a stand-in for the CUDA runtime (tests/fake_cuda.cpp)."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "gale_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+PRELUDE = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <thread>
+#include <vector>
+#include "gg_handle.h"
+#include "gg_kernels.cuh"
+extern std::atomic<int> f_registers, f_unregisters, f_copies, f_syncs;
+extern std::atomic<bool> f_refuse_register;
+struct FakeStream { int device; };
+using namespace gg;
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::exit(1); } } while (0)
+constexpr size_t MB = size_t(1) << 20;
+struct H1 {  // a handle on a device
+    FakeStream s;
+    Handle H;
+    explicit H1(int dev = 0) : s{dev} {
+        H.stream = reinterpret_cast<cudaStream_t>(&s);
+        H.device = dev;
+        copy_handle_created();
+    }
+    ~H1() { H.stream = nullptr; copy_handle_destroyed(); }
+};
+static void fill(std::vector<char>& v, unsigned seed) {
+    for (size_t i = 0; i < v.size(); i++) v[i] = (char)((i * 2654435761u + seed) >> 13);
+}
+// both ways, compared whole
+static void round_trip(Handle& H, size_t n, unsigned seed) {
+    std::vector<char> a(n), d(n), b(n);
+    fill(a, seed);
+    copy_to_device(H, d.data(), a.data(), n);
+    CHECK(d == a);
+    copy_to_host(H, b.data(), d.data(), n);
+    CHECK(b == a);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    cxx = shutil.which("g++")
+    if cxx is None or not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
+        pytest.skip("no host compiler or no CUDA headers")
+    d = tmp_path_factory.mktemp("copy")
+    flags = [cxx, "-std=c++17", "-O1", "-pthread", "-I", os.path.join(CUDA, "include"), "-I", CSRC, "-include", "atomic",
+             *("-D__d%s_rn(a,b)=((a)%s(b))" % f for f in (("add", "+"), ("sub", "-"), ("mul", "*"), ("div", "/")))]
+    subprocess.run([*flags, "-x", "c++", "-c", os.path.join(CSRC, "gg_copy.cu"), "-o", str(d / "copy.o")], check=True)
+    subprocess.run([*flags, "-c", os.path.join(HERE, "fake_cuda.cpp"), "-o", str(d / "fake.o")], check=True)
+
+    def run(name, body):
+        src = d / (name + ".cpp")
+        src.write_text(PRELUDE + "int main() {\n" + body + "\nreturn 0;\n}\n")
+        exe = str(d / name)
+        subprocess.run([*flags, str(src), str(d / "copy.o"), str(d / "fake.o"), "-o", exe], check=True)
+        r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+def test_handle_of_another_device(host):
+    """A thread whose current device is not the handle's: the events of its slots would belong
+    to the wrong device, so the copy goes the plain way and succeeds."""
+    host("device", """
+        H1 h(1);
+        for (size_t n : {4 * MB, 32 * MB}) round_trip(h.H, n, 1);
+        cudaSetDevice(1);
+        for (size_t n : {4 * MB, 32 * MB}) round_trip(h.H, n, 2);
+    """)
