@@ -193,6 +193,7 @@ constexpr int kMaxDevices = 64;
 struct PerDevice {
     std::mutex mu;  // held for the length of a staged transfer
     Stager* stager = nullptr;
+    bool refused = false;  // the slots could not be had: not tried again while handles live
 };
 // Never destroyed: threads may still wait on a stager when the process exits.
 PerDevice& per_device(int dev) {
@@ -220,11 +221,12 @@ bool staged(Handle& H, void* host, void* device, size_t bytes, bool to_host) {
     PerDevice& D = per_device(dev);
     std::unique_lock<std::mutex> lk(D.mu, std::try_to_lock);
     if (!lk.owns_lock()) return false;
+    if (D.refused) return false;
     if (!D.stager) {
         Stager* s = new (std::nothrow) Stager(dev);
-        if (!s) return false;
-        if (!s->start()) {
+        if (!s || !s->start()) {
             delete s;
+            D.refused = true;
             return false;
         }
         D.stager = s;
@@ -257,6 +259,7 @@ void copy_handle_destroyed() {
         std::lock_guard<std::mutex> lk2(D.mu);
         delete D.stager;
         D.stager = nullptr;
+        D.refused = false;
     }
 }
 

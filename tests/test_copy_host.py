@@ -78,3 +78,22 @@ def test_handle_of_another_device(host):
         cudaSetDevice(1);
         for (size_t n : {4 * MB, 32 * MB}) round_trip(h.H, n, 2);
     """)
+
+
+def test_refused_slots_are_not_asked_for_again(host):
+    """Where the slots cannot be registered, one attempt is made while any handle lives."""
+    host("refused", """
+        f_refuse_register = true;
+        {
+            H1 a, b;
+            for (int k = 0; k < 6; k++) round_trip(k & 1 ? a.H : b.H, 64 * MB + 4097 * k, k);
+            CHECK(f_registers == 1 && f_unregisters == 0);
+        }
+        f_refuse_register = false;
+        {
+            H1 a;
+            for (int k = 0; k < 3; k++) round_trip(a.H, 64 * MB, k);
+            CHECK(f_registers == 2);
+        }
+        CHECK(f_unregisters == 1);
+    """)
