@@ -11,15 +11,19 @@
 // the last of them to wake).
 //
 // The slots (kWorkers · 2 · kSlot = 16 MB of pinned memory per device) and the threads are
-// shared by the process, made by the first large transfer and given back when the last handle is
-// destroyed.  One transfer uses them at a time; one that finds them busy (another thread's
-// handle) takes the plain copy, so no caller waits for another.
+// shared by the process, made once the transfers have earned them and given back when the last
+// handle is destroyed.  One transfer uses them at a time; one that finds them busy (another
+// thread's handle) takes the plain copy, so no caller waits for another.
 //
 // A program that keeps one handle at a time pays for the slots with each, so they have to
 // be cheap: pinned pages of 4 KB cost 12-25 ms for 32 MB (cudaMallocHost) and 3-11 ms to
-// give back, huge pages registered in place 3-4 and 0.8 ms for 16 MB.  Slots of 0.25 / 0.5 /
-// 1 / 2 MB moved the cells in 1.8 / 1.5 / 1.3 / 1.3 ms and the coordinates in 13.5 / 11.4 /
-// 9.5 / 10.4 ms, device work included.
+// give back, huge pages registered in place 3-4 and 0.8 ms for 16 MB.  And they have to be
+// worth it: a handle that located 270 k points and was destroyed took 4.5 ms with slots made
+// for its 1.1 MB of cells, 2.1 without.  Staging gains some 0.1-0.15 µs per KB read back into
+// fresh memory and a fifth of that on the way up, so the slots are made when the bytes
+// down and a quarter of the bytes up since the last handle-free moment pass kEarn.
+// Slots of 0.25 / 0.5 / 1 / 2 MB moved 28 MB of cells in 1.8 / 1.5 / 1.3 / 1.3 ms and 170 MB
+// of coordinates in 13.5 / 11.4 / 9.5 / 10.4 ms, device work included.
 #include <sys/mman.h>
 
 #include <algorithm>
@@ -46,6 +50,7 @@ static_assert(kSlots % kHugePage == 0, "the slots are whole huge pages");
 constexpr size_t kMinChunk = size_t(128) << 10;
 constexpr size_t kMinOut = size_t(1) << 20;   // to the host: the page faults alone pay for the threads
 constexpr size_t kMinIn = size_t(12) << 20;   // to the device: the driver stages 3-10 MB as fast (0.34-1.06 ms), 21 MB in 2.2 ms against 1.7
+constexpr size_t kEarn = size_t(16) << 20;
 
 struct Job {
     char* host = nullptr;
@@ -193,6 +198,7 @@ constexpr int kMaxDevices = 64;
 struct PerDevice {
     std::mutex mu;  // held for the length of a staged transfer
     Stager* stager = nullptr;
+    size_t earned = 0;     // of kEarn, by transfers that took the plain copy for want of slots
     bool refused = false;  // the slots could not be had: not tried again while handles live
 };
 // Never destroyed: threads may still wait on a stager when the process exits.
@@ -223,6 +229,8 @@ bool staged(Handle& H, void* host, void* device, size_t bytes, bool to_host) {
     if (!lk.owns_lock()) return false;
     if (D.refused) return false;
     if (!D.stager) {
+        D.earned += to_host ? bytes : bytes / 4;
+        if (D.earned < kEarn) return false;
         Stager* s = new (std::nothrow) Stager(dev);
         if (!s || !s->start()) {
             delete s;
@@ -259,6 +267,7 @@ void copy_handle_destroyed() {
         std::lock_guard<std::mutex> lk2(D.mu);
         delete D.stager;
         D.stager = nullptr;
+        D.earned = 0;
         D.refused = false;
     }
 }

@@ -97,3 +97,57 @@ def test_refused_slots_are_not_asked_for_again(host):
         }
         CHECK(f_unregisters == 1);
     """)
+
+
+def test_slots_are_made_when_the_transfers_have_earned_them(host):
+    """16 MB down, or 64 MB up, or a sum of both; not for a handle that moves less, whatever
+    its predecessors moved; given back with the last handle."""
+    host("earned", """
+        std::vector<char> a(64 * MB), b(64 * MB);
+        for (int k = 0; k < 5; k++) {  // handles one after the other, 12 MB each
+            H1 h;
+            for (int t = 0; t < 3; t++) copy_to_host(h.H, a.data(), b.data(), 4 * MB);
+            copy_to_host(h.H, a.data(), b.data(), MB - 1);  // too small to count
+            copy_to_device(h.H, a.data(), b.data(), 12 * MB - 1);
+        }
+        CHECK(f_registers == 0);
+        {
+            H1 h;
+            for (int t = 0; t < 4; t++) {
+                CHECK(f_registers == 0);
+                copy_to_host(h.H, a.data(), b.data(), 4 * MB);
+            }
+            CHECK(f_registers == 1);
+            round_trip(h.H, 20 * MB + 5, 1);
+            CHECK(f_registers == 1);
+        }
+        CHECK(f_unregisters == 1);
+        {
+            H1 h;
+            copy_to_device(h.H, a.data(), b.data(), 63 * MB);
+            CHECK(f_registers == 1);
+            copy_to_device(h.H, a.data(), b.data(), 12 * MB);
+            CHECK(f_registers == 2);
+        }
+        {
+            H1 h;
+            copy_to_host(h.H, a.data(), b.data(), 16 * MB);
+            CHECK(f_registers == 3);
+        }
+        CHECK(f_unregisters == 3);
+    """)
+
+
+def test_threads_on_both_ways(host):
+    """Transfers of several handles at once, uploads above their threshold among them: one has
+    the slots, the others copy, and every array arrives whole."""
+    host("threads", """
+        H1 h[4];
+        std::vector<std::thread> ts;
+        for (int k = 0; k < 4; k++)
+            ts.emplace_back([&, k] {
+                for (int t = 0; t < 12; t++) round_trip(h[k].H, 12 * MB + 77773 * (k + 4 * t) - 1, k + t);
+            });
+        for (auto& t : ts) t.join();
+        CHECK(f_registers == 1);
+    """)
