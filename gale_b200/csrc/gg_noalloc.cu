@@ -40,9 +40,10 @@ __global__ void k_scan_add(int32_t* __restrict__ out, int64_t n, const int32_t* 
 void launch_scatter(int64_t np, int64_t nel, uint32_t* cell, const int32_t* offsets, const int32_t* place,
                     int32_t* unsorted, cudaStream_t st);
 template <bool kInPlace>
-__global__ void k_segsort(int64_t nel, const int32_t* __restrict__ offsets, int32_t* unsorted, int32_t* perm,
+__global__ void k_segsort(int64_t nel, int per, const int32_t* __restrict__ offsets, int32_t* unsorted, int32_t* perm,
                           int32_t* flags);
-int segsort_grid(int64_t nel);
+int segsort_per(int64_t np, int64_t nel);
+int segsort_grid(int64_t nel, int per);
 
 namespace {
 
@@ -161,7 +162,8 @@ extern "C" GG_API int gg_locate_noalloc(const gg_mesh_desc* mesh, int64_t n_poin
     // the points' places ride in d_cell above the element (k_locate), no second count
     launch_scatter(n_points, nel, d_cell, d_offsets, nullptr, d_order, st);
     if (!launched("gg_locate_noalloc: launch of the scatter failed")) return GG_ERR_CUDA;
-    k_segsort<true><<<segsort_grid(nel), kSegBlock, 0, st>>>(nel, d_offsets, d_order, d_order, flags);
+    const int per = segsort_per(n_points, nel);
+    k_segsort<true><<<segsort_grid(nel, per), kSegBlock, 0, st>>>(nel, per, d_offsets, d_order, d_order, flags);
     if (!launched("gg_locate_noalloc: launch of the per-element sort failed")) return GG_ERR_CUDA;
     int32_t hflags[2] = {0, 0};
     if (cudaMemcpyAsync(hflags, flags, sizeof(hflags), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -205,32 +205,34 @@ __device__ __forceinline__ void sort_segment(int32_t* seg, int n) {
         if (j < n) seg[j] = v[j];
 }
 
-// Every element's point indices ascending (they are distinct).  A block takes 128 elements:
-// their contiguous range passes through shared memory and one thread sorts each element with
-// a network in registers, 191 compare-exchanges for up to 32 points.  One warp per element
-// ranking each index against all others took 300 µs for 28.3 M points on 2^20 elements
-// (issue-bound); the network needs a tenth of the instructions and leaves the two passes
-// over the indices.  Blocks with an element of more than 64 points or a range beyond
-// kSegCap rank them by warps instead.
+// Every element's point indices ascending (they are distinct).  A block takes `per` elements
+// (at most 128, one per thread): where each holds at most 64 points, their contiguous range
+// passes through shared memory and one thread sorts each element with a network in registers,
+// 191 compare-exchanges for up to 32 points.  One warp per element ranking each index against
+// all others took 300 µs for 28.3 M points on 2^20 elements (issue-bound); the network needs a
+// tenth of the instructions and leaves the two passes over the indices.  Blocks with a larger
+// element or a range beyond kSegCap rank them, a warp per element; the ranking is
+// quadratic, so a block then wants few elements (segsort_per).
 // kInPlace: perm is unsorted, elements beyond kPlaceSort points are left alone and counted in
 // flags[1].  Otherwise unsorted is overwritten with the sorted points' element.
 template <bool kInPlace>
 __global__ void __launch_bounds__(kSegBlock)
-k_segsort(int64_t nel, const int32_t* __restrict__ offsets, int32_t* unsorted, int32_t* perm, int32_t* flags) {
+k_segsort(int64_t nel, int per, const int32_t* __restrict__ offsets, int32_t* unsorted, int32_t* perm, int32_t* flags) {
     __shared__ int32_t buf[kSegCap];
     __shared__ int s_most[kSegBlock / 32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    for (int64_t e0 = (int64_t)blockIdx.x * kSegBlock; e0 < nel; e0 += (int64_t)gridDim.x * kSegBlock) {
-        const int64_t e = e0 + threadIdx.x, e1 = e0 + kSegBlock < nel ? e0 + kSegBlock : nel;
+    for (int64_t e0 = (int64_t)blockIdx.x * per; e0 < nel; e0 += (int64_t)gridDim.x * per) {
+        const int64_t e = e0 + threadIdx.x, e1 = e0 + per < nel ? e0 + per : nel;
         const int32_t r0 = offsets[e0], r1 = offsets[e1];
-        const int32_t b = e < nel ? offsets[e] : r1, n = e < nel ? offsets[e + 1] - b : 0;
+        const int32_t b = e < e1 ? offsets[e] : r1, n = e < e1 ? offsets[e + 1] - b : 0;
         const int most_w = __reduce_max_sync(0xffffffffu, n);
         if (lane == 0) s_most[wib] = most_w;
         __syncthreads();
         int most = 0;
 #pragma unroll
         for (int w = 0; w < kSegBlock / 32; w++) most = max(most, s_most[w]);
-        if (most <= 64 && r1 - r0 <= kSegCap) {
+        // (few threads sort in a block of few elements: from 33 points on its warps rank faster)
+        if (most <= (per < kSegBlock / 2 ? 32 : 64) && r1 - r0 <= kSegCap) {
             for (int32_t i = r0 + threadIdx.x; i < r1; i += kSegBlock) buf[i - r0] = unsorted[i];
             __syncthreads();
             int32_t* seg = buf + (b - r0);
@@ -249,34 +251,51 @@ k_segsort(int64_t nel, const int32_t* __restrict__ offsets, int32_t* unsorted, i
             int32_t* mine = buf + wib * kPlaceSort;
             for (int64_t q = e0 + wib; q < e1; q += kSegBlock / 32) {
                 const int32_t qb = offsets[q], qn = offsets[q + 1] - qb;
-                if (kInPlace && qn > kPlaceSort) {
-                    if (lane == 0) atomicAdd(&flags[1], 1);
-                    continue;
-                }
-                const int32_t* from = unsorted + qb;
-                if (kInPlace) {
+                if (qn <= kPlaceSort) {
                     for (int k = lane; k < qn; k += 32) mine[k] = unsorted[qb + k];
                     __syncwarp();
-                    from = mine;
-                }
-                for (int k = lane; k < qn; k += 32) {
-                    const int32_t v = from[k];
-                    int rank = 0;
-                    for (int j = 0; j < qn; j++) rank += (from[j] < v);
-                    perm[qb + rank] = v;
+                    for (int k = lane; k < qn; k += 32) {
+                        const int32_t v = mine[k];
+                        int rank = 0;
+                        for (int j = 0; j < qn; j++) rank += (mine[j] < v);
+                        perm[qb + rank] = v;
+                    }
+                } else if (kInPlace) {
+                    if (lane == 0) atomicAdd(&flags[1], 1);
+                    continue;
+                } else {
+                    for (int k = lane; k < qn; k += 32) {
+                        const int32_t v = unsorted[qb + k];
+                        int rank = 0;
+                        for (int j = 0; j < qn; j++) rank += (unsorted[qb + j] < v);
+                        perm[qb + rank] = v;
+                    }
                 }
                 __syncwarp();
                 if (!kInPlace)
                     for (int k = lane; k < qn; k += 32) unsorted[qb + k] = (int32_t)q;
+                __syncwarp();
             }
         }
         __syncthreads();
     }
 }
-template __global__ void k_segsort<true>(int64_t, const int32_t* __restrict__, int32_t*, int32_t*, int32_t*);
+template __global__ void k_segsort<true>(int64_t, int, const int32_t* __restrict__, int32_t*, int32_t*, int32_t*);
 
-int segsort_grid(int64_t nel) {
-    const int64_t g = (nel + kSegBlock - 1) / kSegBlock, cap = 32 * (int64_t)num_sms();
+// Elements per block of k_segsort.  Above 40 points on average many elements exceed what the
+// network takes: one per warp (µs of a location, 128 / 4 per block: 64² of 64 120 / 74, of 300
+// 871 / 160, 16² of 1000 7273 / 352); on meshes that leave the SMs idle from 32 points on (16³
+// of 40 68 / 60).  Below, a warp's worth at least: large meshes in blocks of 128, smaller ones
+// on four blocks per SM (64² of 20 in blocks of 4: 59 µs, of 32 and 128: 50).
+int segsort_per(int64_t np, int64_t nel) {
+    if (np > 40 * nel || (np > 32 * nel && nel < 32 * (int64_t)num_sms())) return kSegBlock / 32;
+    int per = kSegBlock;
+    while (per > 32 && nel < (int64_t)per * 4 * num_sms()) per /= 2;
+    return per;
+}
+
+int segsort_grid(int64_t nel, int per) {
+    const int64_t g = (nel + per - 1) / per, cap = 32 * (int64_t)num_sms();
     return (int)(g < 1 ? 1 : g < cap ? g : cap);
 }
 
@@ -383,8 +402,9 @@ int64_t locate_and_sort(Handle& H) {
     // cell_s holds the unsorted permutation until k_segsort overwrites it
     launch_scatter(np, nel, H.cell.as<uint32_t>(), H.offsets.as<int32_t>(), H.perm.as<int32_t>(),
                    H.cell_s.as<int32_t>(), st);
-    k_segsort<false><<<segsort_grid(nel), kSegBlock, 0, st>>>(nel, H.offsets.as<int32_t>(), H.cell_s.as<int32_t>(),
-                                                              H.perm.as<int32_t>(), nullptr);
+    const int per = segsort_per(np, nel);
+    k_segsort<false><<<segsort_grid(nel, per), kSegBlock, 0, st>>>(nel, per, H.offsets.as<int32_t>(),
+                                                                   H.cell_s.as<int32_t>(), H.perm.as<int32_t>(), nullptr);
     GG_CUDA(cudaGetLastError());
     int32_t outside = 0;
     GG_CUDA(cudaMemcpyAsync(&outside, H.flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
