@@ -15,9 +15,13 @@ namespace gg {
 
 namespace {
 
-template <int DIM>
+constexpr int64_t kPackPoints = 1 << 20;  // points × dim from which the velocities are packed
+
+// kPacked: u holds the components of a node side by side (k_node_velocity), else vector after
+// vector
+template <int DIM, bool kPacked>
 __device__ bool velocity_at(const MeshK& mk, const double* x, const double2* __restrict__ axes,
-                            const double2* __restrict__ u, double* v) {
+                            const double* __restrict__ u, double* v) {
     int inds[3] = {0, 0, 0};
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
@@ -53,11 +57,17 @@ __device__ bool velocity_at(const MeshK& mk, const double* x, const double2* __r
 #pragma unroll
         for (int d = 0; d < DIM; d++) N *= 1.0 + (((a >> d) & 1) ? xi[d] : -xi[d]);
         const int32_t n = n0 + (a & 1) + ((a >> 1) & 1) * mk.nn[0] + (DIM == 3 ? ((a >> 2) & 1) * mk.nn[0] * mk.nn[1] : 0);
-        double uc[4];
-        const double2 u01 = u[(int64_t)n * (DIM - 1)];
-        uc[0] = u01.x;
-        uc[1] = u01.y;
-        if (DIM == 3) uc[2] = u[(int64_t)n * (DIM - 1) + 1].x;
+        double uc[3];
+        if constexpr (kPacked) {
+            const double2* un = reinterpret_cast<const double2*>(u) + (int64_t)n * (DIM - 1);
+            const double2 u01 = un[0];
+            uc[0] = u01.x;
+            uc[1] = u01.y;
+            if (DIM == 3) uc[2] = un[1].x;
+        } else {
+#pragma unroll
+            for (int c = 0; c < DIM; c++) uc[c] = u[(int64_t)c * mk.nnode + n];
+        }
 #pragma unroll
         for (int c = 0; c < DIM; c++) v[c] += uc[c] * N;
     }
@@ -80,16 +90,16 @@ __global__ void k_node_velocity(int64_t nnode, const double* __restrict__ u, dou
 // sector of its own.  With the components in separate vectors a 3D stage read 24 of them per
 // point; a node's components in one 32-byte sector make it 8 (7.1 M points, two stages:
 // 978 → 639 µs).
-template <int DIM>
+template <int DIM, bool kPacked>
 __global__ void k_advect(MeshK mk, int64_t np, double dt, int order, const double2* __restrict__ axes,
-                         const double2* __restrict__ u, double* __restrict__ coords, int32_t* __restrict__ flag) {
+                         const double* __restrict__ u, double* __restrict__ coords, int32_t* __restrict__ flag) {
     const double hdt = __dmul_rn(0.5, dt);
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np;
          p += (int64_t)gridDim.x * blockDim.x) {
         double x0[3], x[3], k1[3], k2[3];
 #pragma unroll
         for (int c = 0; c < DIM; c++) x0[c] = coords[p * DIM + c];
-        if (!velocity_at<DIM>(mk, x0, axes, u, k1)) {
+        if (!velocity_at<DIM, kPacked>(mk, x0, axes, u, k1)) {
             atomicAdd(flag, 1);
             continue;
         }
@@ -99,7 +109,7 @@ __global__ void k_advect(MeshK mk, int64_t np, double dt, int order, const doubl
         } else {
 #pragma unroll
             for (int c = 0; c < DIM; c++) x[c] = __dadd_rn(x0[c], __dmul_rn(hdt, k1[c]));
-            if (velocity_at<DIM>(mk, x, axes, u, k2)) {
+            if (velocity_at<DIM, kPacked>(mk, x, axes, u, k2)) {
 #pragma unroll
                 for (int c = 0; c < DIM; c++) x[c] = __dadd_rn(x0[c], __dmul_rn(dt, k2[c]));
             } else {
@@ -120,15 +130,26 @@ int advect(Handle& H, double dt, int order, const double* d_u, double* d_out) {
     GG_CUDA(cudaMemsetAsync(H.flag.p, 0, sizeof(int32_t) * 4, H.stream));
     const int g = grid_for(H.np, 256);
     const double2* axes = element_axes(H);
-    H.adv_u.ensure(sizeof(double2) * H.nnode * (H.dim - 1));
-    double2* un = H.adv_u.as<double2>();
-    const int gn = grid_for(H.nnode, 256);
-    if (H.dim == 2) {
-        k_node_velocity<2><<<gn, 256, 0, H.stream>>>(H.nnode, d_u, un);
-        k_advect<2><<<g, 256, 0, H.stream>>>(H.mk, H.np, dt, order, axes, un, H.coords.as<double>(), H.flag.as<int32_t>());
+    auto move = [&](auto kernel, const void* u) {
+        kernel<<<g, 256, 0, H.stream>>>(H.mk, H.np, dt, order, axes, static_cast<const double*>(u), H.coords.as<double>(),
+                                        H.flag.as<int32_t>());
+    };
+    // Packing is a launch of its own, which small swarms do not earn back (µs per call, packed /
+    // by component: 64² of 60 50 / 46, 128² of 20 67 / 65, 256×64 of 40 70 / 76, 16³ of 27 58 / 48)
+    if (H.np * H.dim < kPackPoints) {
+        if (H.dim == 2) move(k_advect<2, false>, d_u);
+        else move(k_advect<3, false>, d_u);
     } else {
-        k_node_velocity<3><<<gn, 256, 0, H.stream>>>(H.nnode, d_u, un);
-        k_advect<3><<<g, 256, 0, H.stream>>>(H.mk, H.np, dt, order, axes, un, H.coords.as<double>(), H.flag.as<int32_t>());
+        H.adv_u.ensure(sizeof(double2) * H.nnode * (H.dim - 1));
+        double2* un = H.adv_u.as<double2>();
+        const int gn = grid_for(H.nnode, 256);
+        if (H.dim == 2) {
+            k_node_velocity<2><<<gn, 256, 0, H.stream>>>(H.nnode, d_u, un);
+            move(k_advect<2, true>, un);
+        } else {
+            k_node_velocity<3><<<gn, 256, 0, H.stream>>>(H.nnode, d_u, un);
+            move(k_advect<3, true>, un);
+        }
     }
     GG_CUDA(cudaGetLastError());
     int32_t bad = 0;
