@@ -9,9 +9,13 @@
 // moments, points and vectors of big meshes) still use cudaMalloc / cudaFree directly.
 // Chunks stay with the process until it exits.
 //
+// An allocation that finds the device full takes back the scratch that handles of the same
+// device keep between their calls (PointScratch) and tries once more.
+//
 // Reuse is as safe as with cudaFree, which synchronises the device: a block goes back on its
 // free list only after cudaDeviceSynchronize, so no kernel of any stream still uses it when
 // another handle is given it.
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -45,37 +49,97 @@ int size_class(size_t bytes) {
     return s;
 }
 
+// Every handle's scratch.  Never destroyed, as the pools.
+struct ScratchList {
+    std::mutex mu;
+    std::vector<PointScratch*> all;
+};
+ScratchList& scratch_list() {
+    static ScratchList* l = new ScratchList;
+    return *l;
+}
+
+// Give back the idle scratch on this device; a set in use (by this thread's own call too) stays.
+bool reclaim_scratch(int dev) {
+    ScratchList& L = scratch_list();
+    std::lock_guard<std::mutex> lk(L.mu);
+    bool any = false;
+    for (PointScratch* s : L.all) {
+        if (s->busy.exchange(true, std::memory_order_acquire)) continue;
+        for (int k = 0; DBuf* b = s->all(k); k++)
+            if (b->p && b->dev == dev) {
+                b->release();
+                any = true;
+            }
+        s->busy.store(false, std::memory_order_release);
+    }
+    return any;
+}
+
+void* device_malloc(size_t bytes, int dev) {
+    void* p = nullptr;
+    cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && reclaim_scratch(dev)) {
+        cudaGetLastError();
+        p = nullptr;
+        e = cudaMalloc(&p, bytes);
+    }
+    GG_CUDA(e);
+    return p;
+}
+
 }  // namespace
+
+PointScratch::PointScratch() {
+    ScratchList& L = scratch_list();
+    std::lock_guard<std::mutex> lk(L.mu);
+    L.all.push_back(this);
+}
+
+PointScratch::~PointScratch() {
+    ScratchList& L = scratch_list();
+    std::lock_guard<std::mutex> lk(L.mu);
+    L.all.erase(std::find(L.all.begin(), L.all.end(), this));
+}
 
 void* dev_alloc(size_t bytes, int* dev_out) {
     int dev = 0;
     GG_CUDA(cudaGetDevice(&dev));
     *dev_out = dev;
-    if (bytes > (size_t(1) << kMaxShift) || dev < 0 || dev >= kMaxDevices) {
-        void* p = nullptr;
-        GG_CUDA(cudaMalloc(&p, bytes));
-        return p;
-    }
+    if (bytes > (size_t(1) << kMaxShift) || dev < 0 || dev >= kMaxDevices) return device_malloc(bytes, dev);
     const int s = size_class(bytes);
     const size_t sz = size_t(1) << s;
     DevicePool& P = pool(dev);
-    std::lock_guard<std::mutex> lk(P.mu);
-    std::vector<void*>& fl = P.free_list[s];
-    if (!fl.empty()) {
-        void* p = fl.back();
-        fl.pop_back();
-        return p;
+    for (bool retry = false;; retry = true) {
+        {
+            std::lock_guard<std::mutex> lk(P.mu);
+            std::vector<void*>& fl = P.free_list[s];
+            if (!fl.empty()) {
+                void* p = fl.back();
+                fl.pop_back();
+                return p;
+            }
+            if (P.left < sz) {  // the rest of the current chunk (< 4 MB) is left unused
+                void* c = nullptr;
+                const cudaError_t e = cudaMalloc(&c, kChunk);
+                if (e == cudaSuccess) {
+                    P.cur = static_cast<char*>(c);
+                    P.left = kChunk;
+                } else if (retry || e != cudaErrorMemoryAllocation) {
+                    GG_CUDA(e);
+                } else {
+                    cudaGetLastError();
+                }
+            }
+            if (P.left >= sz) {
+                void* p = P.cur;
+                P.cur += sz;
+                P.left -= sz;
+                return p;
+            }
+        }
+        reclaim_scratch(dev);  // without the lock: small scratch goes back to this pool
     }
-    if (P.left < sz) {  // the rest of the current chunk (< 4 MB) is left unused
-        void* c = nullptr;
-        GG_CUDA(cudaMalloc(&c, kChunk));
-        P.cur = static_cast<char*>(c);
-        P.left = kChunk;
-    }
-    void* p = P.cur;
-    P.cur += sz;
-    P.left -= sz;
-    return p;
 }
 
 void dev_free(void* p, size_t bytes, int dev) {

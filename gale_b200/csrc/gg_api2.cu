@@ -448,7 +448,8 @@ int gg_get_integration_points(gg_handle* h, double* xi, double* weight) {
     Handle& H = h->H;
     if (!H.located) return gg::err(H, GG_ERR_STATE, "gg_locate has not succeeded");
     GG_TRY2(h, {
-        DBuf &dx = H.int_xi, &dw = H.int_w;
+        PointScratch::Use use(H.point_scratch);
+        DBuf &dx = H.point_scratch.int_xi, &dw = H.point_scratch.int_w;
         dx.ensure(sizeof(double) * H.np * H.dim);
         dw.ensure(sizeof(double) * H.np);
         gg::k_int_points<<<gg::grid_for(H.np, 256), 256, 0, H.stream>>>(

@@ -1110,7 +1110,9 @@ int dvc_update(Handle& H, const gg_pcdvc_params* prm, gg_pcdvc_stats* stats) {
         return GG_OK;
     }
     // point order: keep flags, integration points
-    DBuf &keep_p = H.pc_keep, &newidx = H.pc_newidx, &xi_p = H.pc_xi_p, &w_p = H.pc_w_p;
+    PointScratch& P = H.point_scratch;
+    PointScratch::Use use(P);
+    DBuf &keep_p = P.keep, &newidx = P.newidx, &xi_p = P.xi_p, &w_p = P.w_p;
     keep_p.ensure(sizeof(int32_t) * np);
     newidx.ensure(sizeof(int32_t) * (np + 1));
     xi_p.ensure(sizeof(double) * np * dim);
@@ -1121,7 +1123,7 @@ int dvc_update(Handle& H, const gg_pcdvc_params* prm, gg_pcdvc_stats* stats) {
     int32_t nsurv = 0;
     exclusive_scan_i32(H, keep_p.as<int32_t>(), newidx.as<int32_t>(), np, H.scan_tmp, &nsurv);
     const int64_t np2 = (int64_t)nsurv + nsplit_tot;
-    DBuf &coords2 = H.pc_coords, &mat2 = H.pc_mat, &ps2 = H.pc_ps, &xi2 = H.pc_xi, &w2 = H.pc_w;
+    DBuf &coords2 = P.coords, &mat2 = P.mat, &ps2 = P.ps, &xi2 = P.xi, &w2 = P.w;
     coords2.ensure(sizeof(double) * np2 * dim);
     mat2.ensure(sizeof(int32_t) * np2);
     ps2.ensure(sizeof(double) * np2);

@@ -3,9 +3,11 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <map>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "gg_internal.cuh"
@@ -47,6 +49,46 @@ struct DBuf {
     }
     template <class T>
     T* as() const { return static_cast<T*>(p); }
+};
+
+// Per-point scratch of population control and of the integration points' read-back, kept
+// from call to call because cudaMalloc and cudaFree of it cost more than the work (2.7 M points
+// in 3D: 5 ms kept, 20-70 ms allocated anew).  In 3D it is 140 bytes per point beside some 160 that
+// are in use, so it is only lent: a call that runs out of device memory takes the idle scratch of
+// every handle of its device back (gg_alloc.cu), and beyond kKeep nothing is kept.
+struct PointScratch {
+    static constexpr size_t kKeep = size_t(1) << 30;
+    // population control: point-order arrays and the other half of the point set it swaps in
+    DBuf keep, newidx, xi_p, w_p, coords, mat, ps, xi, w;
+    DBuf int_xi, int_w;  // integration points in point order (gg_get_integration_points)
+    std::atomic<bool> busy{false};
+    PointScratch();
+    ~PointScratch();
+    DBuf* all(int k) {
+        DBuf* b[] = {&keep, &newidx, &xi_p, &w_p, &coords, &mat, &ps, &xi, &w, &int_xi, &int_w};
+        return k < (int)(sizeof b / sizeof b[0]) ? b[k] : nullptr;
+    }
+    size_t held() {
+        size_t n = 0;
+        for (int k = 0; DBuf* b = all(k); k++) n += b->bytes;
+        return n;
+    }
+    void release() {
+        for (int k = 0; DBuf* b = all(k); k++) b->release();
+    }
+    // Held for the length of a call that uses the buffers.
+    struct Use {
+        PointScratch& s;
+        explicit Use(PointScratch& s_) : s(s_) {
+            while (s.busy.exchange(true, std::memory_order_acquire)) std::this_thread::yield();
+        }
+        ~Use() {
+            if (s.held() > kKeep) s.release();
+            s.busy.store(false, std::memory_order_release);
+        }
+        Use(const Use&) = delete;
+        Use& operator=(const Use&) = delete;
+    };
 };
 
 // One multigrid level (level 0 = the fine mesh).
@@ -96,9 +138,7 @@ struct Handle {
     gg_weights weights{GG_WEIGHTS_CONSTANT, {10, 10, 10}};
     bool dvc_valid = false;
     DBuf w_s, xi_pts, dvc_defer, dvc_cent, dvc_keep, dvc_err, dvc_nsplit, dvc_ndel, dvc_parent, dvc_new, dvc_scan, dvc_scan2;
-    // population control's point-order scratch and the other half of the point set it swaps in
-    DBuf pc_keep, pc_newidx, pc_xi_p, pc_w_p, pc_coords, pc_mat, pc_ps, pc_xi, pc_w;
-    DBuf int_xi, int_w;  // integration points in point order (gg_get_integration_points)
+    PointScratch point_scratch;
 
     // operator
     DBuf mom64, mom32, kdiag64, kdiag32, sdiag, hvec, f;

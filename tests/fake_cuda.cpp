@@ -1,11 +1,13 @@
-// A host-only stand-in for the CUDA runtime calls of gg_copy.cu: copies happen at once, every
-// handle remembers its device, and calls can be told to fail.
+// A host-only stand-in for the CUDA runtime calls of gg_copy.cu and gg_alloc.cu: copies happen
+// at once, events and streams remember their device, the device has as much memory as a test
+// says, and calls can be told to fail.
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cstdlib>
 #include <cstring>
-
-#include "gg_handle.h"
+#include <map>
+#include <mutex>
 
 std::atomic<int> f_device{0}, f_registers{0}, f_unregisters{0}, f_copies{0}, f_syncs{0};
 std::atomic<bool> f_refuse_register{false};
@@ -14,7 +16,29 @@ thread_local int t_device = 0;
 struct FakeEvent { int device; };
 struct FakeStream { int device; };
 
+// device memory: blocks of their true size, backed by 16 bytes
+std::mutex f_mu;
+std::map<void*, size_t> f_blocks;
+size_t f_capacity = size_t(1) << 40, f_used = 0;
+
+#undef cudaMalloc
 extern "C" {
+cudaError_t cudaMalloc(void** p, size_t n) {
+    std::lock_guard<std::mutex> lk(f_mu);
+    if (f_used + n > f_capacity) return cudaErrorMemoryAllocation;
+    *p = std::malloc(16);
+    f_blocks[*p] = n;
+    f_used += n;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    std::lock_guard<std::mutex> lk(f_mu);
+    f_used -= f_blocks.at(p);
+    f_blocks.erase(p);
+    std::free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = t_device; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { t_device = d; return cudaSuccess; }
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
@@ -46,8 +70,3 @@ cudaError_t cudaMemcpyAsync(void* to, const void* from, size_t n, cudaMemcpyKind
     return cudaSuccess;
 }
 }
-
-namespace gg {
-void* dev_alloc(size_t, int*) { return nullptr; }
-void dev_free(void*, size_t, int) {}
-}  // namespace gg

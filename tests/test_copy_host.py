@@ -1,5 +1,6 @@
-"""The host side of the staged transfers (gale_b200/csrc/gg_copy.cu) on the CPU: the file
-compiled for the host against a stand-in for the CUDA runtime (tests/fake_cuda.cpp)."""
+"""The host side of the staged transfers (gale_b200/csrc/gg_copy.cu) and of the device memory
+behind the handles (gg_alloc.cu) on the CPU: the files compiled for the host against a
+stand-in for the CUDA runtime (tests/fake_cuda.cpp)."""
 import os
 import shutil
 import subprocess
@@ -19,6 +20,7 @@ PRELUDE = r"""
 #include "gg_kernels.cuh"
 extern std::atomic<int> f_registers, f_unregisters, f_copies, f_syncs;
 extern std::atomic<bool> f_refuse_register;
+extern size_t f_capacity, f_used;
 struct FakeStream { int device; };
 using namespace gg;
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::exit(1); } } while (0)
@@ -56,14 +58,16 @@ def host(tmp_path_factory):
     d = tmp_path_factory.mktemp("copy")
     flags = [cxx, "-std=c++17", "-O1", "-pthread", "-I", os.path.join(CUDA, "include"), "-I", CSRC, "-include", "atomic",
              *("-D__d%s_rn(a,b)=((a)%s(b))" % f for f in (("add", "+"), ("sub", "-"), ("mul", "*"), ("div", "/")))]
-    subprocess.run([*flags, "-x", "c++", "-c", os.path.join(CSRC, "gg_copy.cu"), "-o", str(d / "copy.o")], check=True)
+    for f in ("gg_copy", "gg_alloc"):
+        subprocess.run([*flags, "-x", "c++", "-c", os.path.join(CSRC, f + ".cu"), "-o", str(d / (f + ".o"))], check=True)
     subprocess.run([*flags, "-c", os.path.join(HERE, "fake_cuda.cpp"), "-o", str(d / "fake.o")], check=True)
+    objs = [str(d / f) for f in ("gg_copy.o", "gg_alloc.o", "fake.o")]
 
     def run(name, body):
         src = d / (name + ".cpp")
         src.write_text(PRELUDE + "int main() {\n" + body + "\nreturn 0;\n}\n")
         exe = str(d / name)
-        subprocess.run([*flags, str(src), str(d / "copy.o"), str(d / "fake.o"), "-o", exe], check=True)
+        subprocess.run([*flags, str(src), *objs, "-o", exe], check=True)
         r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
         assert r.returncode == 0, r.stdout + r.stderr
     return run
@@ -150,4 +154,78 @@ def test_threads_on_both_ways(host):
             });
         for (auto& t : ts) t.join();
         CHECK(f_registers == 1);
+    """)
+
+
+def test_kept_point_scratch_is_lent(host):
+    """Scratch that a handle keeps between calls is taken back when any handle of its device
+    needs the memory, not while a call uses it, not from another device; beyond its bound it
+    is not kept at all."""
+    host("scratch", """
+        const size_t GB = size_t(1) << 30;
+        f_capacity = 4 * GB;
+        H1 a, b;
+        {
+            PointScratch::Use use(a.H.point_scratch);
+            a.H.point_scratch.coords.ensure(600 * MB);
+            a.H.point_scratch.int_w.ensure(300 * MB);
+            a.H.point_scratch.keep.ensure(MB);  // from the pool
+        }
+        CHECK(a.H.point_scratch.held() == 901 * MB);  // kept
+        DBuf x;
+        x.ensure(3 * GB);  // fits beside it
+        CHECK(a.H.point_scratch.held() == 901 * MB);
+        {
+            PointScratch::Use use(a.H.point_scratch);
+            DBuf y;
+            bool refused = false;
+            try { y.ensure(600 * MB); } catch (const CudaError&) { refused = true; }
+            CHECK(refused && a.H.point_scratch.held() == 901 * MB);  // in use: not taken
+        }
+        cudaSetDevice(1);
+        {
+            DBuf y;
+            bool refused = false;
+            try { y.ensure(600 * MB); } catch (const CudaError&) { refused = true; }
+            CHECK(refused && a.H.point_scratch.held() == 901 * MB);  // another device's
+        }
+        cudaSetDevice(0);
+        DBuf y;
+        y.ensure(600 * MB);  // by a handle or buffer that knows nothing of it
+        CHECK(a.H.point_scratch.held() == 0 && y.p);
+        y.release();
+        x.release();
+        const size_t before = f_used;
+        {
+            PointScratch::Use use(b.H.point_scratch);
+            b.H.point_scratch.coords.ensure(GB);
+            CHECK(b.H.point_scratch.held() == GB);
+        }
+        CHECK(b.H.point_scratch.held() == GB);
+        {
+            PointScratch::Use use(b.H.point_scratch);
+            b.H.point_scratch.xi.ensure(8 * MB);
+        }
+        CHECK(b.H.point_scratch.held() == 0 && f_used == before);
+    """)
+
+
+def test_pool_chunk_takes_lent_scratch_back(host):
+    """The same for a small buffer whose pool needs a new chunk, with small scratch that goes
+    back to that pool."""
+    host("chunk", """
+        f_capacity = 200 * MB;
+        H1 a;
+        {
+            PointScratch::Use use(a.H.point_scratch);
+            a.H.point_scratch.coords.ensure(100 * MB);
+            a.H.point_scratch.ps.ensure(3 * MB);
+        }
+        DBuf small[40];
+        for (int k = 0; k < 16; k++) small[k].ensure(4 * MB - 1);  // the first chunk, and one block too many
+        CHECK(a.H.point_scratch.held() == 0);
+        for (int k = 16; k < 32; k++) small[k].ensure(4 * MB - 1);  // the second chunk and the returned block
+        bool refused = false;
+        try { small[32].ensure(4 * MB); small[33].ensure(200 * MB); } catch (const CudaError&) { refused = true; }
+        CHECK(refused);
     """)
