@@ -3,27 +3,27 @@
 // The caller's arrays are pageable, and a cudaMemcpyAsync on pageable memory is staged by
 // the driver on the calling thread: 170 MB of advected coordinates took 35 ms (5 GB/s,
 // mostly page faults of the freshly allocated result), 28 MB of owning cells 1.6 ms, beside
-// 1 ms and 0.5 ms of device work.  Transfers of kMinOut or kMinIn bytes and more are cut into chunks that
-// kWorkers threads move through pinned slots: each thread copies its own chunks between the
-// caller's memory and its two slots (the page faults then spread over the threads) while
-// the copy engine moves the other slot, all on the handle's stream.  The coordinates took
-// 9.8 ms, the cells 1.1 ms; 14 threads gained nothing on either (a transfer then waits for
-// the last of them to wake).
+// 1 ms and 0.5 ms of device work.  Transfers of kMinOut or kMinIn bytes and more are cut into
+// chunks that kWorkers threads move through pinned slots: each thread copies its own chunks
+// between the caller's memory and its two slots (the page faults then spread over the threads)
+// while the copy engine moves the other slot, all on the handle's stream.  14 threads gained
+// nothing (a transfer then waits for the last of them to wake).
 //
-// The slots (kWorkers · 2 · kSlot = 16 MB of pinned memory per device) and the threads are
-// shared by the process, made once the transfers have earned them and given back when the last
-// handle is destroyed.  One transfer uses them at a time; one that finds them busy (another
-// thread's handle) takes the plain copy, so no caller waits for another.
+// The slots (two per thread, pinned) and the threads are shared by the process, made once the
+// transfers have earned them and given back when the last handle is destroyed.  One transfer
+// uses them at a time; one that finds them busy (another thread's handle) takes the plain copy,
+// so no caller waits for another.
 //
 // A program that keeps one handle at a time pays for the slots with each, so they have to
-// be cheap: pinned pages of 4 KB cost 12-25 ms for 32 MB (cudaMallocHost) and 3-11 ms to
-// give back, huge pages registered in place 3-4 and 0.8 ms for 16 MB.  And they have to be
-// worth it: a handle that located 270 k points and was destroyed took 4.5 ms with slots made
-// for its 1.1 MB of cells, 2.1 without.  Staging gains some 0.1-0.15 µs per KB read back into
-// fresh memory and a fifth of that on the way up, so the slots are made when the bytes
-// down and a quarter of the bytes up since the last handle-free moment pass kEarn.
-// Slots of 0.25 / 0.5 / 1 / 2 MB moved 28 MB of cells in 1.8 / 1.5 / 1.3 / 1.3 ms and 170 MB
-// of coordinates in 13.5 / 11.4 / 9.5 / 10.4 ms, device work included.
+// be cheap: pinned pages of 4 KB cost 3.1 ms for 4 MB (cudaMallocHost) and 0.6 to give back, huge
+// pages registered in place 0.55 and 0.25 (16 MB: 1.3-2.4 and 0.5).  And they have to be
+// worth it: a handle that located 270 k points and was destroyed took 4.5 ms with 16 MB of slots
+// made for its 1.1 MB of cells, 2.1 without.  The plain copy takes 0.22 µs per KB into fresh huge
+// pages and 0.45 into small ones, staging 0.06, and on the way up it gains a quarter of that; so
+// the bytes down and a quarter of the bytes up since no handle was alive are counted,
+// kEarnSmall of them make slots of 256 KB (4 MB) and kEarnLarge slots of 1 MB (16 MB), which move
+// 28 MB of cells in 1.3 ms instead of 1.8 and 170 MB of coordinates in 9.5 instead of 13.5
+// (0.5 MB: 1.5 and 11.4; 2 MB: 1.3 and 10.4; device work included).
 #include <sys/mman.h>
 
 #include <algorithm>
@@ -43,14 +43,13 @@ namespace gg {
 namespace {
 
 constexpr int kWorkers = 8;
-constexpr size_t kSlot = size_t(1) << 20;
+constexpr size_t kSlotSmall = size_t(256) << 10, kSlotLarge = size_t(1) << 20;
 constexpr size_t kHugePage = size_t(2) << 20;
-constexpr size_t kSlots = kSlot * 2 * kWorkers;
-static_assert(kSlots % kHugePage == 0, "the slots are whole huge pages");
+static_assert(kSlotSmall * 2 * kWorkers % kHugePage == 0, "the slots are whole huge pages");
 constexpr size_t kMinChunk = size_t(128) << 10;
 constexpr size_t kMinOut = size_t(1) << 20;   // to the host: the page faults alone pay for the threads
 constexpr size_t kMinIn = size_t(12) << 20;   // to the device: the driver stages 3-10 MB as fast (0.34-1.06 ms), 21 MB in 2.2 ms against 1.7
-constexpr size_t kEarn = size_t(16) << 20;
+constexpr size_t kEarnSmall = size_t(8) << 20, kEarnLarge = size_t(128) << 20;
 
 struct Job {
     char* host = nullptr;
@@ -62,7 +61,9 @@ struct Job {
 
 // The slots, their events and the threads of one device.
 struct Stager {
-    int dev;
+    const int dev;
+    const size_t slot;  // bytes of one of the 2·kWorkers slots
+    const size_t all = slot * 2 * kWorkers;
     void* map = MAP_FAILED;  // the slots, with room to align them
     char* slots = nullptr;
     cudaEvent_t ev[kWorkers][2] = {};
@@ -75,15 +76,15 @@ struct Stager {
     Job job;
     cudaError_t err = cudaSuccess;
 
-    explicit Stager(int d) : dev(d) {}
+    Stager(int d, size_t slot_bytes) : dev(d), slot(slot_bytes) {}
 
     bool start() {
-        map = mmap(nullptr, kSlots + kHugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        map = mmap(nullptr, all + kHugePage, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
         if (map == MAP_FAILED) return false;
         const uintptr_t up = (reinterpret_cast<uintptr_t>(map) + kHugePage - 1) & ~(uintptr_t)(kHugePage - 1);
         slots = reinterpret_cast<char*>(up);
-        madvise(slots, kSlots, MADV_HUGEPAGE);  // refused: pages of 4 KB, which only cost time
-        if (cudaHostRegister(slots, kSlots, cudaHostRegisterPortable) != cudaSuccess) {
+        madvise(slots, all, MADV_HUGEPAGE);  // refused: pages of 4 KB, which only cost time
+        if (cudaHostRegister(slots, all, cudaHostRegisterPortable) != cudaSuccess) {
             cudaGetLastError();
             slots = nullptr;
             return false;
@@ -113,7 +114,7 @@ struct Stager {
             for (auto& x : e)
                 if (x) cudaEventDestroy(x);
         if (slots) cudaHostUnregister(slots);
-        if (map != MAP_FAILED) munmap(map, kSlots + kHugePage);
+        if (map != MAP_FAILED) munmap(map, all + kHugePage);
     }
 
     void loop(int w) {
@@ -137,12 +138,12 @@ struct Stager {
     cudaError_t part(int w) {
         const Job& j = job;
         const size_t n = (j.bytes + j.chunk - 1) / j.chunk;
-        char* slot[2] = {slots + (size_t)(2 * w) * kSlot, slots + (size_t)(2 * w + 1) * kSlot};
+        char* at[2] = {slots + (size_t)(2 * w) * slot, slots + (size_t)(2 * w + 1) * slot};
         auto size = [&](size_t k) { return std::min(j.chunk, j.bytes - k * j.chunk); };
         cudaError_t e = cudaSuccess;
         if (j.to_host) {
             auto issue = [&](size_t k, int s) {
-                e = cudaMemcpyAsync(slot[s], j.device + k * j.chunk, size(k), cudaMemcpyDeviceToHost, j.stream);
+                e = cudaMemcpyAsync(at[s], j.device + k * j.chunk, size(k), cudaMemcpyDeviceToHost, j.stream);
                 if (e == cudaSuccess) e = cudaEventRecord(ev[w][s], j.stream);
                 return e == cudaSuccess;
             };
@@ -153,7 +154,7 @@ struct Stager {
                 const cudaError_t es = cudaEventSynchronize(ev[w][s]);
                 if (e == cudaSuccess) e = es;
                 ok = ok && es == cudaSuccess;
-                if (ok) std::memcpy(j.host + k * j.chunk, slot[s], size(k));
+                if (ok) std::memcpy(j.host + k * j.chunk, at[s], size(k));
             }
         } else {
             int s = 0;
@@ -161,8 +162,8 @@ struct Stager {
             for (size_t k = w; k < n && e == cudaSuccess; k += kWorkers, s ^= 1) {
                 if (used[s]) e = cudaEventSynchronize(ev[w][s]);
                 if (e != cudaSuccess) break;
-                std::memcpy(slot[s], j.host + k * j.chunk, size(k));
-                e = cudaMemcpyAsync(j.device + k * j.chunk, slot[s], size(k), cudaMemcpyHostToDevice, j.stream);
+                std::memcpy(at[s], j.host + k * j.chunk, size(k));
+                e = cudaMemcpyAsync(j.device + k * j.chunk, at[s], size(k), cudaMemcpyHostToDevice, j.stream);
                 if (e == cudaSuccess) e = cudaEventRecord(ev[w][s], j.stream);
                 used[s] = true;
             }
@@ -198,7 +199,7 @@ constexpr int kMaxDevices = 64;
 struct PerDevice {
     std::mutex mu;  // held for the length of a staged transfer
     Stager* stager = nullptr;
-    size_t earned = 0;     // of kEarn, by transfers that took the plain copy for want of slots
+    size_t earned = 0;     // bytes down and a quarter of the bytes up
     bool refused = false;  // the slots could not be had: not tried again while handles live
 };
 // Never destroyed: threads may still wait on a stager when the process exits.
@@ -228,10 +229,13 @@ bool staged(Handle& H, void* host, void* device, size_t bytes, bool to_host) {
     std::unique_lock<std::mutex> lk(D.mu, std::try_to_lock);
     if (!lk.owns_lock()) return false;
     if (D.refused) return false;
-    if (!D.stager) {
-        D.earned += to_host ? bytes : bytes / 4;
-        if (D.earned < kEarn) return false;
-        Stager* s = new (std::nothrow) Stager(dev);
+    D.earned += to_host ? bytes : bytes / 4;
+    const size_t slot = D.earned >= kEarnLarge ? kSlotLarge : kSlotSmall;
+    if (!D.stager && D.earned < kEarnSmall) return false;
+    if (!D.stager || D.stager->slot < slot) {
+        delete D.stager;
+        D.stager = nullptr;
+        Stager* s = new (std::nothrow) Stager(dev, slot);
         if (!s || !s->start()) {
             delete s;
             D.refused = true;
@@ -245,7 +249,7 @@ bool staged(Handle& H, void* host, void* device, size_t bytes, bool to_host) {
     j.bytes = bytes;
     // every thread gets work, in chunks large enough to pay for their calls
     size_t c = (bytes / (2 * kWorkers) + 4095) & ~size_t(4095);
-    j.chunk = c < kMinChunk ? kMinChunk : (c > kSlot ? kSlot : c);
+    j.chunk = c < kMinChunk ? kMinChunk : (c > D.stager->slot ? D.stager->slot : c);
     j.to_host = to_host;
     j.stream = H.stream;
     GG_CUDA(D.stager->run(j));

@@ -19,7 +19,7 @@ struct FakeStream { int device; };
 // device memory: blocks of their true size, backed by 16 bytes
 std::mutex f_mu;
 std::map<void*, size_t> f_blocks;
-size_t f_capacity = size_t(1) << 40, f_used = 0;
+size_t f_capacity = size_t(1) << 40, f_used = 0, f_registered = 0;
 
 #undef cudaMalloc
 extern "C" {
@@ -48,8 +48,9 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
     a->type = cudaMemoryTypeUnregistered;
     return cudaSuccess;
 }
-cudaError_t cudaHostRegister(void*, size_t, unsigned) {
+cudaError_t cudaHostRegister(void*, size_t n, unsigned) {
     f_registers++;
+    f_registered = n;
     return f_refuse_register ? cudaErrorMemoryAllocation : cudaSuccess;
 }
 cudaError_t cudaHostUnregister(void*) { f_unregisters++; return cudaSuccess; }

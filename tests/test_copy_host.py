@@ -20,7 +20,7 @@ PRELUDE = r"""
 #include "gg_kernels.cuh"
 extern std::atomic<int> f_registers, f_unregisters, f_copies, f_syncs;
 extern std::atomic<bool> f_refuse_register;
-extern size_t f_capacity, f_used;
+extern size_t f_capacity, f_used, f_registered;
 struct FakeStream { int device; };
 using namespace gg;
 #define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::exit(1); } } while (0)
@@ -96,7 +96,7 @@ def test_refused_slots_are_not_asked_for_again(host):
         f_refuse_register = false;
         {
             H1 a;
-            for (int k = 0; k < 3; k++) round_trip(a.H, 64 * MB, k);
+            for (int k = 0; k < 3; k++) round_trip(a.H, 24 * MB, k);
             CHECK(f_registers == 2);
         }
         CHECK(f_unregisters == 1);
@@ -104,13 +104,14 @@ def test_refused_slots_are_not_asked_for_again(host):
 
 
 def test_slots_are_made_when_the_transfers_have_earned_them(host):
-    """16 MB down, or 64 MB up, or a sum of both; not for a handle that moves less, whatever
-    its predecessors moved; given back with the last handle."""
+    """Small slots from 8 MB down, or 32 MB up, or a sum of both, large ones from 128 MB; none
+    for a handle that moves less, whatever its predecessors moved; given back with the last
+    handle."""
     host("earned", """
-        std::vector<char> a(64 * MB), b(64 * MB);
-        for (int k = 0; k < 5; k++) {  // handles one after the other, 12 MB each
+        std::vector<char> a(128 * MB), b(128 * MB);
+        for (int k = 0; k < 5; k++) {  // handles one after the other, 5 MB each
             H1 h;
-            for (int t = 0; t < 3; t++) copy_to_host(h.H, a.data(), b.data(), 4 * MB);
+            for (int t = 0; t < 2; t++) copy_to_host(h.H, a.data(), b.data(), 5 * MB / 2);
             copy_to_host(h.H, a.data(), b.data(), MB - 1);  // too small to count
             copy_to_device(h.H, a.data(), b.data(), 12 * MB - 1);
         }
@@ -119,26 +120,30 @@ def test_slots_are_made_when_the_transfers_have_earned_them(host):
             H1 h;
             for (int t = 0; t < 4; t++) {
                 CHECK(f_registers == 0);
-                copy_to_host(h.H, a.data(), b.data(), 4 * MB);
+                copy_to_host(h.H, a.data(), b.data(), 2 * MB);
             }
+            CHECK(f_registers == 1 && f_registered == 4 * MB);
+            round_trip(h.H, 60 * MB + 5, 1);
             CHECK(f_registers == 1);
-            round_trip(h.H, 20 * MB + 5, 1);
-            CHECK(f_registers == 1);
-        }
-        CHECK(f_unregisters == 1);
-        {
-            H1 h;
-            copy_to_device(h.H, a.data(), b.data(), 63 * MB);
-            CHECK(f_registers == 1);
-            copy_to_device(h.H, a.data(), b.data(), 12 * MB);
+            copy_to_host(h.H, a.data(), b.data(), 50 * MB);  // 133 MB by now
+            CHECK(f_registers == 2 && f_unregisters == 1 && f_registered == 16 * MB);
+            round_trip(h.H, 33 * MB + 4099, 2);
             CHECK(f_registers == 2);
         }
+        CHECK(f_unregisters == 2);
         {
             H1 h;
-            copy_to_host(h.H, a.data(), b.data(), 16 * MB);
-            CHECK(f_registers == 3);
+            copy_to_device(h.H, a.data(), b.data(), 31 * MB);
+            CHECK(f_registers == 2);
+            copy_to_device(h.H, a.data(), b.data(), 12 * MB);
+            CHECK(f_registers == 3 && f_registered == 4 * MB);
         }
-        CHECK(f_unregisters == 3);
+        {
+            H1 h;
+            copy_to_host(h.H, a.data(), b.data(), 128 * MB);
+            CHECK(f_registers == 4 && f_registered == 16 * MB);
+        }
+        CHECK(f_unregisters == 4);
     """)
 
 
@@ -153,7 +158,7 @@ def test_threads_on_both_ways(host):
                 for (int t = 0; t < 12; t++) round_trip(h[k].H, 12 * MB + 77773 * (k + 4 * t) - 1, k + t);
             });
         for (auto& t : ts) t.join();
-        CHECK(f_registers == 1);
+        CHECK(f_registers == 2 && f_unregisters == 1);  // small, then large slots
     """)
 
 
