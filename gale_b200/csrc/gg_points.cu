@@ -231,8 +231,8 @@ k_segsort(int64_t nel, int per, const int32_t* __restrict__ offsets, int32_t* un
         int most = 0;
 #pragma unroll
         for (int w = 0; w < kSegBlock / 32; w++) most = max(most, s_most[w]);
-        // (few threads sort in a block of few elements: from 33 points on its warps rank faster)
-        if (most <= (per < kSegBlock / 2 ? 32 : 64) && r1 - r0 <= kSegCap) {
+        // (in a block of a few elements hardly a thread sorts: from 33 points on its warps rank faster)
+        if (most <= (per < 32 ? 32 : 64) && r1 - r0 <= kSegCap) {
             for (int32_t i = r0 + threadIdx.x; i < r1; i += kSegBlock) buf[i - r0] = unsorted[i];
             __syncthreads();
             int32_t* seg = buf + (b - r0);
@@ -285,12 +285,13 @@ template __global__ void k_segsort<true>(int64_t, int, const int32_t* __restrict
 // Elements per block of k_segsort.  Above 40 points on average many elements exceed what the
 // network takes: one per warp (µs of a location, 128 / 4 per block: 64² of 64 120 / 74, of 300
 // 871 / 160, 16² of 1000 7273 / 352); on meshes that leave the SMs idle from 32 points on (16³
-// of 40 68 / 60).  Below, a warp's worth at least: large meshes in blocks of 128, smaller ones
+// of 40 68 / 60), and always on those of up to four elements per SM.  Below, a warp's worth at least: large meshes in blocks of 128, smaller ones
 // on four blocks per SM (64² of 20 in blocks of 4: 59 µs, of 32 and 128: 50).
 int segsort_per(int64_t np, int64_t nel) {
-    if (np > 40 * nel || (np > 32 * nel && nel < 32 * (int64_t)num_sms())) return kSegBlock / 32;
+    const int64_t sms = num_sms();
+    if (np > 40 * nel || (np > 32 * nel && nel < 32 * sms) || nel <= 4 * sms) return kSegBlock / 32;
     int per = kSegBlock;
-    while (per > 32 && nel < (int64_t)per * 4 * num_sms()) per /= 2;
+    while (per > 32 && nel < per * 4 * sms) per /= 2;
     return per;
 }
 
