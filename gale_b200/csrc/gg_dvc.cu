@@ -395,14 +395,24 @@ __device__ void dvc_element(const DvcArgs& a, DvcSmem& S, int64_t e) {
     }
 }
 
-// the elements k_dvc_group deferred: defer[0] of them, from defer[1]
+// the elements k_dvc_group deferred: defer[0] of them, from defer[2], taken by the warps as they
+// come free (defer[1]); every element where there is no list
 template <int DIM>
-__global__ void __launch_bounds__(32 * kWarps) k_dvc(DvcArgs a, const int32_t* __restrict__ defer) {
+__global__ void __launch_bounds__(32 * kWarps) k_dvc(DvcArgs a, int32_t* defer) {
     extern __shared__ unsigned char smem_raw[];
     DvcSmem& S = reinterpret_cast<DvcSmem*>(smem_raw)[threadIdx.x >> 5];
-    const int32_t count = defer[0];
-    for (int32_t q = (int32_t)blockIdx.x * kWarps + (threadIdx.x >> 5); q < count; q += (int32_t)gridDim.x * kWarps) {
-        dvc_element<DIM>(a, S, defer[1 + q]);
+    const int lane = threadIdx.x & 31;
+    const int32_t count = defer ? defer[0] : (int32_t)a.nel;
+    int32_t q = (int32_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (defer && (int32_t)blockIdx.x * kWarps >= count) return;
+    for (;;) {
+        if (defer) {
+            if (lane == 0) q = atomicAdd(&defer[1], 1);
+            q = __shfl_sync(0xffffffffu, q, 0);
+        }
+        if (q >= count) return;
+        dvc_element<DIM>(a, S, defer ? defer[2 + q] : q);
+        if (!defer) return;
         __syncwarp();
     }
 }
@@ -428,11 +438,13 @@ struct DvcGroup {
     int ring;          // ring entries, a power of two ≥ the grid cells
     int xi_at, owner_at, mark_at, ring_at, len_at, list_at, stride;  // byte layout of an element
     uint32_t mnx, mny; // ⌈65536/nx⌉, ⌈65536/ny⌉: c/nx = c·mnx >> 16 exactly for c < 1024, nx ≤ 64
-    int32_t* defer;    // [0] count, then the elements left to k_dvc
+    int32_t* defer;    // [0] count, [1] taken, then the elements left to k_dvc
 };
 constexpr int kGroupPts = 64;       // points per element: one 64-bit mask
 constexpr int kGroupThreads = 128;
 constexpr int kGroupPasses = 1024;
+template <int DIM>
+constexpr int kRingMax = DIM == 3 ? 2048 : 1024;
 
 template <int DIM>
 __device__ __forceinline__ void cell_ijk(const DvcArgs& a, const DvcGroup& f, int c, int& i, int& j, int& k) {
@@ -807,7 +819,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_dvc_group(DvcArgs a, DvcGroup
         }
     }
     if (defer) {
-        if (own && gl == 0) f.defer[1 + atomicAdd(&f.defer[0], 1)] = (int32_t)e;
+        if (own && gl == 0) f.defer[2 + atomicAdd(&f.defer[0], 1)] = (int32_t)e;
         return;
     }
     for (int k = gl; k < m; k += G) {
@@ -834,8 +846,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_dvc_group(DvcArgs a, DvcGroup
     }
 }
 
+// cap: points an element may hold; fill: points of an element as full as they commonly are
 template <int DIM, int G>
-void launch_group(const DvcArgs& a, DvcGroup f, int cap, cudaStream_t st) {
+void launch_group(const DvcArgs& a, DvcGroup f, int cap, int fill, cudaStream_t st) {
     int at = 0;
     auto take = [&](int bytes, int align) {
         at = (at + align - 1) / align * align;
@@ -844,8 +857,16 @@ void launch_group(const DvcArgs& a, DvcGroup f, int cap, cudaStream_t st) {
         return r;
     };
     f.cap = cap;
+    // The ring has to hold every list of a pass at once (and, afterwards, every cell).  In 2D
+    // twice the cells do; in 3D the need grows with the points as well: 5.8 √(points · cells) covers
+    // the largest of 300 random elements each of 12 to 64 points on 4³ to 10³ cells (27 on 10³:
+    // 948 entries, 40: 1132, 64: 1423).  A ring of 1024 made 28 % of elements of 40 points on 10³
+    // cells, and all of 64, grow their diagram twice (16³ elements of some 30: 1.27 ms, 0.51 with
+    // 2048); but one that is larger than it has to be leaves room for fewer elements (32³ of 27:
+    // 2.51 ms with 2048, 2.44 with 1024), so a few fuller elements may exceed it.
+    const double need = DIM == 3 ? 5.8 * sqrt((double)fill * a.ncell) : 0.0;
     int r = 32;
-    while (r < a.ncell || r < 2 * DIM * cap || (r < 2 * a.ncell && r < 512)) r *= 2;
+    while (r < a.ncell || r < 2 * DIM * cap || (r < 2 * a.ncell && r < 512) || (1.1 * r < need && r < kRingMax<DIM>)) r *= 2;
     f.ring = r;
     f.xi_at = take((int)sizeof(double) * DIM * cap, 16);
     f.mark_at = take((a.ncell + 31) / 32 * 4, 4);
@@ -857,31 +878,45 @@ void launch_group(const DvcArgs& a, DvcGroup f, int cap, cudaStream_t st) {
     f.mnx = (65536u + a.nx - 1) / a.nx;
     f.mny = (65536u + a.ny - 1) / a.ny;
     constexpr int per = kGroupThreads / G;
-    // At most 64 points, 1024 cells and a ring of 1024: below the shared memory a kernel may
-    // use without asking.  The limit is state of the function, shared by every host thread, so
-    // nothing sets it to the size of one launch.
-    static_assert(per * (8 * DIM * kGroupPts + kMaxCells / 8 + kMaxCells + 2 * 1024 + 7 * kGroupPts + 48) <= 48 * 1024 - 3 * 8 * kAxis,
+    // Below the shared memory a kernel may use without asking.  That limit is state of the
+    // function, shared by every host thread, so nothing sets it to the size of one launch.
+    static_assert(per * (8 * DIM * kGroupPts + kMaxCells / 8 + kMaxCells + 2 * kRingMax<DIM> + 7 * kGroupPts + 48) <=
+                      48 * 1024 - 3 * 8 * kAxis,
                   "a block of groups fits the default shared memory");
     const size_t smem = (size_t)f.stride * per;
     k_dvc_group<DIM, G><<<(unsigned)((a.nel + per - 1) / per), kGroupThreads, smem, st>>>(a, f);
     GG_CUDA(cudaGetLastError());
 }
 
-// Every element through k_dvc_group, the deferred ones through k_dvc.
+// Every element through k_dvc_group, the deferred ones through k_dvc.  most: points of the
+// fullest element.
 template <int DIM>
-void launch_dvc(const DvcArgs& a, int32_t* defer, cudaStream_t st) {
-    GG_CUDA(cudaMemsetAsync(defer, 0, sizeof(int32_t), st));
-    // room for half again the mean point count: uniform swarms and those PCDVC keeps within
-    // its bounds stay below it, and smaller elements leave room for more of them per SM
-    const double mean = (double)a.np / (double)a.nel;
-    int cap = ((int)(1.5 * mean) + 8 + 7) / 8 * 8;
-    cap = cap > kGroupPts ? kGroupPts : cap;
-    DvcGroup f{};
-    f.defer = defer;
-    launch_group<DIM, DIM == 3 ? 32 : 16>(a, f, cap, st);
+void launch_dvc(const DvcArgs& a, int most, int32_t* defer, cudaStream_t st) {
     const size_t smem = sizeof(DvcSmem) * kWarps;
     GG_CUDA(cudaFuncSetAttribute(k_dvc<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t want = (a.nel + kWarps - 1) / kWarps;
+    const double mean = (double)a.np / (double)a.nel;
+    const int extra = a.pc ? a.max_splits : 0;
+    // k_dvc alone where hardly an element can be small enough for a group, and where all elements
+    // run at once there: a fuller one would then only start when the groups are done (8² of 55
+    // on 10² cells: both 0.42 ms, alone 0.29).  In between both: a clustered swarm has many small
+    // elements whatever its mean (128² of 70 on 30² cells, clustered: both 1.27 ms, alone 11.1).
+    const bool one_wave = want <= 2 * num_sms();
+    if (mean + extra > 2 * kGroupPts || (one_wave && most + extra > kGroupPts)) {
+        k_dvc<DIM><<<(unsigned)want, 32 * kWarps, smem, st>>>(a, nullptr);
+        GG_CUDA(cudaGetLastError());
+        return;
+    }
+    GG_CUDA(cudaMemsetAsync(defer, 0, 2 * sizeof(int32_t), st));
+    // Room for half again the mean point count: uniform swarms and those PCDVC keeps within
+    // its bounds stay below it, and smaller elements leave room for more of them per SM.  A mesh
+    // that does not fill the SMs has room for its fullest element.
+    int cap = one_wave ? (most + extra + 7) / 8 * 8 : ((int)(1.5 * mean) + 8 + 7) / 8 * 8;
+    cap = cap > kGroupPts ? kGroupPts : cap < 8 ? 8 : cap;
+    DvcGroup f{};
+    f.defer = defer;
+    const int fill = std::min({cap, most + extra, (int)(1.15 * mean) + 4});
+    launch_group<DIM, DIM == 3 ? 32 : 16>(a, f, cap, one_wave ? cap : fill, st);
     const int blocks = (int)std::min<int64_t>(want, 2 * num_sms());
     k_dvc<DIM><<<blocks, 32 * kWarps, smem, st>>>(a, defer);
     GG_CUDA(cudaGetLastError());
@@ -1071,11 +1106,11 @@ int dvc_update(Handle& H, const gg_pcdvc_params* prm, gg_pcdvc_stats* stats) {
         a.nsplit = H.dvc_nsplit.as<int32_t>();
         a.ndel = H.dvc_ndel.as<int32_t>();
     }
-    H.dvc_defer.ensure(sizeof(int32_t) * (nel + 1));
+    H.dvc_defer.ensure(sizeof(int32_t) * (nel + 2));
     if (dim == 2)
-        launch_dvc<2>(a, H.dvc_defer.as<int32_t>(), st);
+        launch_dvc<2>(a, H.most_points, H.dvc_defer.as<int32_t>(), st);
     else
-        launch_dvc<3>(a, H.dvc_defer.as<int32_t>(), st);
+        launch_dvc<3>(a, H.most_points, H.dvc_defer.as<int32_t>(), st);
     int32_t err[2] = {0, 0};
     GG_CUDA(cudaMemcpyAsync(err, H.dvc_err.p, sizeof err, cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));

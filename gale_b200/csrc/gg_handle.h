@@ -131,6 +131,7 @@ struct Handle {
     DBuf axes;               // centre and half width of every element per axis
     bool ps_given = false;   // a plastic strain was passed with the points (else it is zero)
     DBuf adv_u;              // velocity per node, padded to whole words of 16 or 32 bytes
+    int32_t most_points = 0;  // points of the fullest element (gg_locate)
     bool located = false;
     // integration weights (gg_dvc.cu): with GG_WEIGHTS_DVC, xi_s holds the Voronoi
     // centroids and w_s the volumes of the sorted points once dvc_valid; xi_pts keeps

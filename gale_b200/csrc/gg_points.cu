@@ -214,7 +214,8 @@ __device__ __forceinline__ void sort_segment(int32_t* seg, int n) {
 // element or a range beyond kSegCap rank them, a warp per element; the ranking is
 // quadratic, so a block then wants few elements (segsort_per).
 // kInPlace: perm is unsorted, elements beyond kPlaceSort points are left alone and counted in
-// flags[1].  Otherwise unsorted is overwritten with the sorted points' element.
+// flags[1].  Otherwise unsorted is overwritten with the sorted points' element, and flags[1]
+// becomes the largest element's count.
 template <bool kInPlace>
 __global__ void __launch_bounds__(kSegBlock)
 k_segsort(int64_t nel, int per, const int32_t* __restrict__ offsets, int32_t* unsorted, int32_t* perm, int32_t* flags) {
@@ -231,6 +232,7 @@ k_segsort(int64_t nel, int per, const int32_t* __restrict__ offsets, int32_t* un
         int most = 0;
 #pragma unroll
         for (int w = 0; w < kSegBlock / 32; w++) most = max(most, s_most[w]);
+        if (!kInPlace && threadIdx.x == 0) atomicMax(&flags[1], most);
         // (in a block of a few elements hardly a thread sorts: from 33 points on its warps rank faster)
         if (most <= (per < 32 ? 32 : 64) && r1 - r0 <= kSegCap) {
             for (int32_t i = r0 + threadIdx.x; i < r1; i += kSegBlock) buf[i - r0] = unsorted[i];
@@ -405,11 +407,14 @@ int64_t locate_and_sort(Handle& H) {
                    H.cell_s.as<int32_t>(), st);
     const int per = segsort_per(np, nel);
     k_segsort<false><<<segsort_grid(nel, per), kSegBlock, 0, st>>>(nel, per, H.offsets.as<int32_t>(),
-                                                                   H.cell_s.as<int32_t>(), H.perm.as<int32_t>(), nullptr);
+                                                                   H.cell_s.as<int32_t>(), H.perm.as<int32_t>(),
+                                                                   H.flag.as<int32_t>());
     GG_CUDA(cudaGetLastError());
-    int32_t outside = 0;
-    GG_CUDA(cudaMemcpyAsync(&outside, H.flag.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    int32_t flags[2] = {0, 0};
+    GG_CUDA(cudaMemcpyAsync(flags, H.flag.p, sizeof flags, cudaMemcpyDeviceToHost, st));
     GG_CUDA(cudaStreamSynchronize(st));
+    const int32_t outside = flags[0];
+    H.most_points = flags[1];
     const int64_t np_in = np - outside;
     k_gather_points<<<grid_for(np_in, 256), 256, 0, st>>>(
         H.mk, np_in, H.perm.as<int32_t>(), H.cell_s.as<int32_t>(), element_axes(H), H.coords.as<double>(),
