@@ -526,6 +526,13 @@ int gg_time_apply(gg_handle* h, int32_t precision, int32_t reps, double* ms_per_
     return GG_OK;
 }
 
+int gg_select_cg64(gg_handle* h, int32_t form) {
+    if (!h) return GG_ERR_INVALID;
+    if (form < 0 || form > 2) return gg::err(h->H, GG_ERR_INVALID, "form of the FP64 CG");
+    h->H.cg64_form = form;
+    return GG_OK;
+}
+
 int gg_get_coarse_inverse(gg_handle* h, int64_t* n, float* inverse, double* op) {
     if (!h || !n) return GG_ERR_INVALID;
     Handle& H = h->H;

@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 
 #include "gg_cluster_addr.h"
 #include "gg_grid.cuh"
@@ -37,6 +38,8 @@ constexpr int kVecBlocks = 592;  // blocks of 256 threads the vector sums are sp
 constexpr int kCluster = 16;
 constexpr int kStripSmem = 222 * 1024;
 constexpr int64_t kTermBytes = int64_t(32) << 20;  // element terms that stay in L2
+// dofs of the solves under way at once from which they fill the GPU as launches
+constexpr int64_t kSharedDofs2 = 1200000, kSharedDofs3 = 800000;
 
 struct Cg64Args {
     MeshK mk;
@@ -799,28 +802,62 @@ bool run_strip(Handle& H, const Cg64Args& A) {
 }
 
 template <int DIM>
-int run(Handle& H, Cg64Args& A) {
-    if (DIM == 2 && run_strip(H, A)) return 0;
+int run(Handle& H, Cg64Args& A, int solves) {
+    if (DIM == 2 && H.cg64_form != 2 && run_strip(H, A)) return 0;
     constexpr int T = cg64_threads<DIM>(), per = T / 256;
     const int work = std::max(A.tiles << DIM, A.vec_blocks);
     const void* fn = (const void*)k_cg64<DIM>;
     int per_sm = 0;
     GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, 0));
     if (per_sm < 1) return 1;
-    const int grid = std::min((work + per - 1) / per, per_sm * num_sms());
+    // its share of the SMs beside other solves, whose grids then run at the same time
+    const int grid = std::min((work + per - 1) / per, std::max(1, per_sm * num_sms() / solves));
     GG_CUDA(cudaMemsetAsync(A.gb, 0, sizeof(GridBarrier), H.stream));
     void* args[] = {(void*)&A};
     GG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(T), args, 0, H.stream));
     return 0;
 }
 
+struct InFlight {
+    std::mutex mu;
+    int solves = 0;
+    int64_t dofs = 0;
+};
+InFlight& in_flight(int dev) {
+    static InFlight f[64];
+    return f[dev >= 0 && dev < 64 ? dev : 0];
+}
+
 }  // namespace
+
+Fp64Flight::Fp64Flight(const Handle& H) : dev(H.device), mine(H.ndof) {
+    InFlight& f = in_flight(dev);
+    std::lock_guard<std::mutex> lk(f.mu);
+    solves = ++f.solves;
+    dofs = f.dofs += mine;
+}
+Fp64Flight::~Fp64Flight() {
+    InFlight& f = in_flight(dev);
+    std::lock_guard<std::mutex> lk(f.mu);
+    f.solves--;
+    f.dofs -= mine;
+}
 
 // x = K⁻¹ b to ‖D⁻¹r‖ ≤ max(rtol‖D⁻¹b‖, 1e-50) in FP64.  Returns 1 when the mesh is outside
 // this kernel's limits (element terms beyond kTermBytes, or a class of more tiles than the
 // class launches have blocks): the caller then runs the captured launches.
-int run_cg64(Handle& H, const double* b, double* x, double rtol, int maxit, int* iters) {
+//
+// Solves from several threads (gg_solve_batch, or a caller's own) share the device.  A
+// cooperative grid on every SM would make them take turns, so each takes its share; and where
+// together they are large enough to fill the GPU, the launches, which interleave freely, do more
+// per second (ms of a batch, launches / turns / shares: 16 of 128² 506 / 466 / 330, of 192² 904 / 1364 /
+// 809, of 24³ 318 / 415 / 292, of 32³ 676 / 886 / 817, 8 of 48³ 1189 / 1460 / 1612, of 400² 2744 /
+// 3094 / 2936; 4 at a time of 32³ 843 / 892 / 728, of 256² 2149 / 2552 / 1636).  The bits are the
+// same in every form.
+int run_cg64(Handle& H, const Fp64Flight& flight, const double* b, double* x, double rtol, int maxit, int* iters) {
     const int dim = H.dim, nc = 1 << dim;
+    if (H.cg64_form == 1 || (H.cg64_form == 0 && flight.solves > 1 && flight.dofs > (dim == 2 ? kSharedDofs2 : kSharedDofs3)))
+        return 1;
     int64_t class_max = 0;
     int tiles = 1;
     for (int c = 0; c < nc; c++) {
@@ -858,7 +895,7 @@ int run_cg64(Handle& H, const double* b, double* x, double rtol, int maxit, int*
     A.gb = reinterpret_cast<GridBarrier*>(A.part_n + 2 * A.vec_blocks);
     A.s = H.scal.as<KrylovScalars>();
     GG_CUDA(cudaMemsetAsync(A.s, 0, sizeof(KrylovScalars), H.stream));
-    if ((dim == 2 ? run<2>(H, A) : run<3>(H, A)) != 0) return 1;
+    if ((dim == 2 ? run<2>(H, A, flight.solves) : run<3>(H, A, flight.solves)) != 0) return 1;
     GG_CUDA(cudaGetLastError());
     H.kernel_launches += 1;
     GG_CUDA(cudaMemcpyAsync(H.h_scal, A.s, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, H.stream));

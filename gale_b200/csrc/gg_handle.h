@@ -153,6 +153,7 @@ struct Handle {
     DBuf u, vstar, ftmp, ub, q, qtmp, r, s;           // FP64
     DBuf cg_b, cg_r, cg_z, cg_p, cg_Ap, cg_x;        // FP64 CG
     DBuf cg_terms, cg_part;                          // its persistent form (gg_cg64.cu)
+    int cg64_form = 0;                                // gg_select_cg64
     DBuf r32, cgr32, z32, p32, Ap32, e32;             // FP32 inner CG
     DBuf scal, red;                                   // KrylovScalars, reduction scratch
     KrylovScalars* h_scal = nullptr;                  // pinned mirror

@@ -108,8 +108,22 @@ bool fused_fcg_enabled();
 // does not apply (the caller runs the host-driven loop), else the solve's status with S's
 // iteration counts, residuals and launch figures filled and H.fail_where set on failure.
 int run_uzawa_fused(Handle& H, const gg_uzawa_params& prm, gg_uzawa_stats& S);
+// A plain FP64 inner solve under way: the solves and their dofs on its device when it began,
+// itself included.
+struct Fp64Flight {
+    int solves = 0;
+    int64_t dofs = 0;
+    explicit Fp64Flight(const Handle& H);
+    ~Fp64Flight();
+    Fp64Flight(const Fp64Flight&) = delete;
+    Fp64Flight& operator=(const Fp64Flight&) = delete;
+
+private:
+    const int dev;
+    const int64_t mine;
+};
 // the plain FP64 Jacobi CG in one launch (gg_cg64.cu); 1: outside its limits
-int run_cg64(Handle& H, const double* b, double* x, double rtol, int maxit, int* iters);
+int run_cg64(Handle& H, const Fp64Flight& flight, const double* b, double* x, double rtol, int maxit, int* iters);
 bool fused_uzawa_enabled();
 // µs per grid barrier of the persistent kernels (measurement, gg_fused.cu)
 int time_grid_barrier(int blocks_per_sm, int iters, double* us);

@@ -607,7 +607,8 @@ int inner_solve(Handle& H, const gg_uzawa_params& prm, const double* b, double* 
     const int64_t nd = H.ndof;
     const uint8_t* bcmask = H.bcmask.as<uint8_t>();
     if (prm.precision == GG_PRECISION_FP64) {
-        const int prc = run_cg64(H, b, x, rtol, maxit, iters);
+        const Fp64Flight flight(H);
+        const int prc = run_cg64(H, flight, b, x, rtol, maxit, iters);
         if (prc != 1) return prc;
         GG_CUDA(cudaMemcpyAsync(H.cg_b.p, b, sizeof(double) * nd, cudaMemcpyDeviceToDevice, H.stream));
         int rc = run_cg<double>(H, "cg64", H.mk, H.mom64.as<double>(), H.kdiag64.as<double>(),

@@ -437,6 +437,12 @@ GG_API int  gg_time_apply(gg_handle* h, int32_t precision, int32_t reps, double*
  * operator replaced by the identity.                                                    */
 GG_API int  gg_get_coarse_inverse(gg_handle* h, int64_t* n, float* inverse, double* op);
 
+/* Inspection (no reference counterpart): the form in which this handle runs its plain FP64
+ * inner solves: 0 chosen by size and by what else runs (the default), 1 the captured class
+ * launches, 2 the cooperative grid also where the cluster form would fit.  Every form gives
+ * the same bits; outside the limits of form 2 the launches run.                           */
+GG_API int  gg_select_cg64(gg_handle* h, int32_t form);
+
 /* Measurement only (no reference counterpart): microseconds per grid barrier of the
  * persistent kernels, `iters` barriers in one cooperative launch of `blocks_per_sm`
  * blocks of 256 threads per SM on the current device (CUDA events, default stream).   */
