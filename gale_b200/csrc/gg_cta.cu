@@ -230,7 +230,7 @@ __device__ __noinline__ double cta_apply2(const MeshK& mk, const float* mom, con
     return en;
 }
 
-// y = K x in FP32 (y zero on entry)
+// y = K x in FP32.  3D adds into y, which has to be zero on entry; 2D writes it whole.
 template <int DIM, bool kEnergy>
 __device__ __forceinline__ double cta_apply32(const CtaLevel& L, const float* x, float* y, float* terms) {
     if constexpr (DIM == 2)

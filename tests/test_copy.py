@@ -40,3 +40,26 @@ def test_two_threads():
     for t in ts:
         t.join()
     assert not fails
+
+
+# coordinates of 16 bytes: 12 MB up, one more and one less, and full large slots; four round trips
+# each, so that the slots are there
+@pytest.mark.parametrize("n", [786_431, 786_432, 786_433, 3_000_001])
+def test_round_trip_staged_both_ways(n):
+    round_trip(n, n, repeat=4)
+
+
+def test_threads_with_staged_uploads():
+    fails = []
+
+    def work(seed):
+        try:
+            round_trip(1_000_001 + seed, seed, repeat=6)
+        except BaseException as e:  # noqa: BLE001
+            fails.append(e)
+    ts = [threading.Thread(target=work, args=(s,)) for s in (1, 2, 3, 4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not fails
