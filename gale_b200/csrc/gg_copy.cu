@@ -24,6 +24,7 @@
 // kEarnSmall of them make slots of 256 KB (4 MB) and kEarnLarge slots of 1 MB (16 MB), which move
 // 28 MB of cells in 1.3 ms instead of 1.8 and 170 MB of coordinates in 9.5 instead of 13.5
 // (0.5 MB: 1.5 and 11.4; 2 MB: 1.3 and 10.4; device work included).
+#include <emmintrin.h>
 #include <sys/mman.h>
 
 #include <algorithm>
@@ -49,7 +50,28 @@ static_assert(kSlotSmall * 2 * kWorkers % kHugePage == 0, "the slots are whole h
 constexpr size_t kMinChunk = size_t(128) << 10;
 constexpr size_t kMinOut = size_t(1) << 20;   // to the host: the page faults alone pay for the threads
 constexpr size_t kMinIn = size_t(12) << 20;   // to the device: the driver stages 3-10 MB as fast (0.34-1.06 ms), 21 MB in 2.2 ms against 1.7
+// Results of this size go past the caches: through them their lines would lie, dirty, in the
+// cores of the threads that wrote them, and the caller's thread would fetch them from there one
+// by one (µs for a transfer into an array in use and a sum over it, plain copy / through the
+// caches / past them: 4 MB 620 / 960 / 602, 8 MB 1220 / 1660 / 1160, 16 MB 2274 / 2180 / 2020).
+// Smaller ones are with the caller's core soon enough (1.5 MB: 281 / 191 / 260), of larger ones the
+// caches keep little (32 MB: 4544 / 3112 / 4160).
+constexpr size_t kPastLo = size_t(7) << 18, kPastHi = size_t(18) << 20;
 constexpr size_t kEarnSmall = size_t(8) << 20, kEarnLarge = size_t(128) << 20;
+
+// memcpy past the caches
+void stream_out(char* to, const char* from, size_t n) {
+    const size_t head = std::min(n, (size_t)(-reinterpret_cast<uintptr_t>(to) & 15));
+    std::memcpy(to, from, head);
+    size_t i = head;
+    for (; i + 64 <= n; i += 64) {
+        __m128i v[4];
+        for (int q = 0; q < 4; q++) v[q] = _mm_loadu_si128(reinterpret_cast<const __m128i*>(from + i + 16 * q));
+        for (int q = 0; q < 4; q++) _mm_stream_si128(reinterpret_cast<__m128i*>(to + i + 16 * q), v[q]);
+    }
+    std::memcpy(to + i, from + i, n - i);
+    _mm_sfence();
+}
 
 struct Job {
     char* host = nullptr;
@@ -142,6 +164,7 @@ struct Stager {
         auto size = [&](size_t k) { return std::min(j.chunk, j.bytes - k * j.chunk); };
         cudaError_t e = cudaSuccess;
         if (j.to_host) {
+            const bool past_caches = j.bytes >= kPastLo && j.bytes < kPastHi;
             auto issue = [&](size_t k, int s) {
                 e = cudaMemcpyAsync(at[s], j.device + k * j.chunk, size(k), cudaMemcpyDeviceToHost, j.stream);
                 if (e == cudaSuccess) e = cudaEventRecord(ev[w][s], j.stream);
@@ -154,7 +177,8 @@ struct Stager {
                 const cudaError_t es = cudaEventSynchronize(ev[w][s]);
                 if (e == cudaSuccess) e = es;
                 ok = ok && es == cudaSuccess;
-                if (ok) std::memcpy(j.host + k * j.chunk, at[s], size(k));
+                if (ok && past_caches) stream_out(j.host + k * j.chunk, at[s], size(k));
+                else if (ok) std::memcpy(j.host + k * j.chunk, at[s], size(k));
             }
         } else {
             int s = 0;

@@ -431,13 +431,13 @@ class StokesProblem:
 
     # diagnostics / operator access
     def point_viscosity(self):
-        eta = np.zeros(self.np)
+        eta = np.empty(self.np)
         self._check(self.lib.gg_get_point_viscosity(self.h, ptr(eta)))
         return eta
 
     def point_yield(self):
-        inc = np.zeros(self.np)
-        y = np.zeros(self.np, dtype=np.uint8)
+        inc = np.empty(self.np)
+        y = np.empty(self.np, dtype=np.uint8)
         self._check(self.lib.gg_get_point_yield(self.h, ptr(inc), ptr(y, C.c_uint8)))
         return inc, y
 
@@ -451,17 +451,17 @@ class StokesProblem:
     def apply_K(self, x, precision="fp64"):
         prec = {"fp64": abi.PRECISION_FP64, "mixed": abi.PRECISION_MIXED}[precision]
         x = f64(x)
-        y = np.zeros_like(x)
+        y = np.empty_like(x)
         self._check(self.lib.gg_apply_K(self.h, prec, ptr(x), ptr(y)))
         return y
 
     def apply_G(self, p):
-        y = np.zeros(self.nnode * self.dim)
+        y = np.empty(self.nnode * self.dim)
         self._check(self.lib.gg_apply_G(self.h, ptr(f64(p)), ptr(y)))
         return y
 
     def apply_GT(self, u):
-        q = np.zeros(self.nel)
+        q = np.empty(self.nel)
         self._check(self.lib.gg_apply_GT(self.h, ptr(f64(u)), ptr(q)))
         return q
 

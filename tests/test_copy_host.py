@@ -14,6 +14,7 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 PRELUDE = r"""
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <thread>
 #include <vector>
 #include "gg_handle.h"
@@ -233,4 +234,23 @@ def test_pool_chunk_takes_lent_scratch_back(host):
         bool refused = false;
         try { small[32].ensure(4 * MB); small[33].ensure(200 * MB); } catch (const CudaError&) { refused = true; }
         CHECK(refused);
+    """)
+
+
+def test_results_past_the_caches_arrive_whole(host):
+    """Sizes around the range that goes past the caches, into arrays at odd addresses, with
+    nothing written outside them."""
+    host("past", """
+        H1 h;
+        std::vector<char> src(33 * MB), dst(33 * MB + 256);
+        fill(src, 3);
+        copy_to_host(h.H, dst.data(), src.data(), 33 * MB);  // the slots are there from now on
+        for (size_t n : {7 * MB / 4 - 1, 7 * MB / 4, 2 * MB + 13, 5 * MB + 63, 18 * MB - 1, 18 * MB, 20 * MB + 1})
+            for (size_t off : {size_t(0), size_t(1), size_t(8), size_t(15), size_t(33)}) {
+                std::memset(dst.data(), 0x5a, n + 256);
+                copy_to_host(h.H, dst.data() + off, src.data() + 7, n);
+                CHECK(std::memcmp(dst.data() + off, src.data() + 7, n) == 0);
+                for (size_t k = 0; k < off; k++) CHECK(dst[k] == 0x5a);
+                for (size_t k = off + n; k < n + 256; k++) CHECK(dst[k] == 0x5a);
+            }
     """)
