@@ -420,19 +420,19 @@ __global__ void __launch_bounds__(32 * kWarps) k_dvc(DvcArgs a, int32_t* defer) 
 // ---- small elements: G lanes per element ---------------------------------------------
 // What bounds the diagrams is the latency of one point's turn (a few dependent
 // shared-memory reads and ballots) times some 200 turns per element, so the time is set by
-// how many elements an SM has in flight.  Here an element takes 2 KB (2D) to 5 KB (3D) of
+// how many elements an SM has in flight.  Here an element takes 2 KB (2D) to 7 KB (3D) of
 // shared memory instead of 36 KB: the boundary lists of successive turns are one ring (a
 // turn's list is consumed before its successor is appended), its claimed cells overwrite
 // the consumed entries, the deduplication is a bitmap cleared after the turn, the points
 // with a list to contest are one 64-bit mask, and a counting sort of the cells by owner
 // (in the ring's memory) replaces a scan of all cells per centroid.  One warp per element
 // with 36 KB each kept 6 elements per SM: 22.4 ms for 32³ elements of 27 points on 10³
-// cells and 4.81 ms for 256×64 of 40 points on 10².  Now 2.34 ms (36 warps per SM, 84 % of
-// the issue slots used: bound by instruction issue) and 0.363 ms.
+// cells and 4.81 ms for 256×64 of 40 points on 10².  Now 2.32 ms (36 warps per SM, 84 % of
+// the issue slots used: bound by instruction issue) and 0.25 ms (76 %).
 // A warp holds 32/G elements that take their turns in lockstep.  A 2D list is a few cells
 // long and a 3D one a few tens, which is where the lanes per element come from: G = 8 / 16 /
-// 32 took 4.37 / 2.51 / 2.34 ms in 3D and 0.338 / 0.363 / 0.583 ms in 2D at 10² cells (16
-// is kept there for finer grids, whose lists are longer).
+// 32 took 4.37 / 2.51 / 2.34 ms in 3D and, with counts that vary, 0.338 / 0.363 / 0.583 ms in
+// 2D at 10² cells (16 is kept there for finer grids, whose lists are longer).
 struct DvcGroup {
     int cap;           // points an element may hold
     int ring;          // ring entries, a power of two ≥ the grid cells
