@@ -224,7 +224,8 @@ struct PerDevice {
     std::mutex mu;  // held for the length of a staged transfer
     Stager* stager = nullptr;
     size_t earned = 0;     // bytes down and a quarter of the bytes up
-    bool refused = false;  // the slots could not be had: not tried again while handles live
+    // slots could not be had (any, or larger ones): not tried again while handles live
+    bool refused = false, keep_small = false;
 };
 // Never destroyed: threads may still wait on a stager when the process exits.
 PerDevice& per_device(int dev) {
@@ -256,16 +257,16 @@ bool staged(Handle& H, void* host, void* device, size_t bytes, bool to_host) {
     D.earned += to_host ? bytes : bytes / 4;
     const size_t slot = D.earned >= kEarnLarge ? kSlotLarge : kSlotSmall;
     if (!D.stager && D.earned < kEarnSmall) return false;
-    if (!D.stager || D.stager->slot < slot) {
-        delete D.stager;
-        D.stager = nullptr;
+    if (!D.stager || (D.stager->slot < slot && !D.keep_small)) {
         Stager* s = new (std::nothrow) Stager(dev, slot);
-        if (!s || !s->start()) {
+        if (s && s->start()) {
+            delete D.stager;
+            D.stager = s;
+        } else {
             delete s;
-            D.refused = true;
-            return false;
+            (D.stager ? D.keep_small : D.refused) = true;
+            if (D.refused) return false;
         }
-        D.stager = s;
     }
     Job j;
     j.host = static_cast<char*>(host);
@@ -296,7 +297,7 @@ void copy_handle_destroyed() {
         delete D.stager;
         D.stager = nullptr;
         D.earned = 0;
-        D.refused = false;
+        D.refused = D.keep_small = false;
     }
 }
 

@@ -104,6 +104,19 @@ def test_refused_slots_are_not_asked_for_again(host):
     """)
 
 
+def test_small_slots_stay_where_large_ones_are_refused(host):
+    host("small", """
+        H1 a;
+        round_trip(a.H, 32 * MB, 1);
+        CHECK(f_registers == 1 && f_registered == 4 * MB);
+        f_refuse_register = true;
+        const int before = f_copies;
+        for (int k = 0; k < 5; k++) round_trip(a.H, 64 * MB, k);
+        CHECK(f_registers == 2 && f_unregisters == 0);       // asked for once
+        CHECK(f_copies - before > 10 * 64 * 4 - 64);         // and every transfer in 256 KB pieces
+    """)
+
+
 def test_slots_are_made_when_the_transfers_have_earned_them(host):
     """Small slots from 8 MB down, or 32 MB up, or a sum of both, large ones from 128 MB; none
     for a handle that moves less, whatever its predecessors moved; given back with the last
