@@ -271,8 +271,9 @@ k_points(MeshK mk, int64_t np, const int32_t* __restrict__ cell_s, const double*
 // ξ-exponent q (every lane the same instructions, with its own power of ξ), lane q the force
 // terms of corners q·NC ….  want_phi 0 / temp null: those weights are zero for every point.
 // Then every lane takes all moments and forms its corners' diagonal terms.
-// Eight elements per warp keep an SM at 32 and more warps, where one thread per element and
-// 39 accumulators left 8; the eight streams of points of a warp meet in L1.
+// Eight elements per warp keep an SM at 20 (FP64, 3D) to 36 warps, where one thread per element
+// and 39 accumulators left 8; the eight streams of points of a warp meet in L1.  Bound by those
+// loads: 48 % of the issue slots, 25 % of the DRAM peak (deeper unrolling changed nothing).
 template <int DIM, typename R, bool kForce>
 __global__ void __launch_bounds__(128)
 k_moments(MeshK mk, int64_t nel, const int32_t* __restrict__ offsets, const double* __restrict__ xi_s, int64_t np,
