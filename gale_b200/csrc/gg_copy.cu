@@ -26,6 +26,7 @@
 // (0.5 MB: 1.5 and 11.4; 2 MB: 1.3 and 10.4; device work included).
 #include <emmintrin.h>
 #include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <condition_variable>
@@ -234,6 +235,7 @@ PerDevice& per_device(int dev) {
 }
 std::mutex g_handles_mu;
 int g_handles = 0;
+pid_t g_pid = 0;  // of the process whose handles these are
 
 bool pageable(const void* host) {
     cudaPointerAttributes a{};
@@ -285,10 +287,11 @@ bool staged(Handle& H, void* host, void* device, size_t bytes, bool to_host) {
 
 void copy_handle_created() {
     std::lock_guard<std::mutex> lk(g_handles_mu);
-    g_handles++;
+    if (g_handles++ == 0) g_pid = getpid();
 }
 
 void copy_handle_destroyed() {
+    if (getpid() != g_pid) return;  // a child of fork: neither the threads nor CUDA came with it
     std::lock_guard<std::mutex> lk(g_handles_mu);
     if (--g_handles > 0) return;
     for (int dev = 0; dev < kMaxDevices; dev++) {

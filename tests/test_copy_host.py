@@ -15,6 +15,8 @@ PRELUDE = r"""
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <sys/wait.h>
+#include <unistd.h>
 #include <thread>
 #include <vector>
 #include "gg_handle.h"
@@ -266,4 +268,27 @@ def test_results_past_the_caches_arrive_whole(host):
                 for (size_t k = 0; k < off; k++) CHECK(dst[k] == 0x5a);
                 for (size_t k = off + n; k < n + 256; k++) CHECK(dst[k] == 0x5a);
             }
+    """)
+
+
+def test_forked_child_drops_its_handles(host):
+    """A child of fork has the handles but not the copy threads: destroying the last handle
+    there returns, and the parent's slots go on."""
+    host("fork", """
+        H1* h = new H1;
+        round_trip(h->H, 32 * MB, 1);
+        CHECK(f_registers == 1);
+        const pid_t pid = fork();
+        if (pid == 0) {
+            alarm(20);  // ends a child that waits for threads it does not have
+            delete h;
+            H1 other;  // nor are there slots for a new one
+            _exit(f_unregisters == 0 ? 0 : 2);
+        }
+        int status = 0;
+        CHECK(waitpid(pid, &status, 0) == pid);
+        CHECK(WIFEXITED(status) && WEXITSTATUS(status) == 0);
+        round_trip(h->H, 32 * MB + 77, 2);
+        delete h;
+        CHECK(f_unregisters == 1);
     """)
